@@ -38,8 +38,17 @@ __host__ __device__ __forceinline__ double from_fx(fx_t v) { return (double)v * 
 __device__ __forceinline__ fx_t to_fxl(double x) { return __double2ll_rn(x * kFxLScale); }
 __host__ __device__ __forceinline__ double from_fxl(fx_t v) { return (double)v * kFxLInv; }
 
+// Seed of a sweep (from the attempt's seed) or of a sub-batch (from its sweep's).
+__host__ __device__ __forceinline__ uint32_t mix_seed(uint32_t a, uint64_t b) {
+    uint64_t x = a * 0x9E3779B97F4A7C15ull ^ (b + 0x632BE59BD9B4E019ull);
+    x ^= x >> 31;
+    x *= 0xBF58476D1CE4E5B9ull;
+    x ^= x >> 29;
+    return (uint32_t)(x ^ (x >> 32));
+}
+
 // p log p with 0 log 0 = 0 (Module.h:23-25).
-__device__ __forceinline__ double plogp(double x) { return x > 0.0 ? x * log(x) : 0.0; }
+__device__ __forceinline__ double plogp(double x) { return x > 0.0 ? __dmul_rn(x, log(x)) : 0.0; }
 
 // Statistics of a module or of a moving unit: flow P, teleport weight TW,
 // dangling flow D and out-flow to other modules OUT. 32 bytes: one sector.
@@ -49,9 +58,13 @@ struct __align__(32) Stat4 {
 
 // Exit flow q = tau (1 - TW) P + (1 - tau) (OUT + (1 - TW) D)
 // (calculateCodeLength, Module.cpp:2978-2991; singleton form Module.cpp:86-95).
+// The rounding of every step is spelt out, here and in the change of a move:
+// left to the compiler, which of two products an addition is fused with
+// depends on the code around it, and decisions that are exact ties would
+// differ between kernels.
 __device__ __forceinline__ double exit_flow(double P, double TW, double D, double OUT) {
-    double e = kAlpha * (1.0 - TW) * P;
-    return e + kBeta * (OUT + (1.0 - TW) * D);
+    const double r = 1.0 - TW;
+    return __fma_rn(__dmul_rn(kAlpha, r), P, __dmul_rn(kBeta, __dadd_rn(OUT, __dmul_rn(r, D))));
 }
 
 __device__ __forceinline__ void atomic_add_fx(fx_t *a, fx_t v) {

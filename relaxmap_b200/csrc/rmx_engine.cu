@@ -254,14 +254,6 @@ __global__ void k_fp64_terms(int32_t n, const double *P, const double *TW, const
     }
 }
 
-__host__ __device__ uint32_t mix_seed(uint32_t a, uint64_t b) {
-    uint64_t x = a * 0x9E3779B97F4A7C15ull ^ (b + 0x632BE59BD9B4E019ull);
-    x ^= x >> 31;
-    x *= 0xBF58476D1CE4E5B9ull;
-    x ^= x >> 29;
-    return (uint32_t)(x ^ (x >> 32));
-}
-
 // ---- a stage loop captured as one graph (while node; the body is one sweep)
 
 // Start of a sweep, as the host loop does it: the sweep number and its seed,
@@ -720,10 +712,12 @@ int64_t rmx_graph::max_degree(const Level &lv) {
 // of lv above the large bin's bound (any sub-batch of the level fits); grown,
 // never shrunk.
 void rmx_graph::ensure_hub_table(const Level &lv) {
+    level_hubs = 0;
     if (lv.n <= 0) return;
     int64_t need[4];
     hub_level_needs(lv, need, dtmp + 12, stream);
     const int64_t units = need[0], parts = need[1], links = need[2], chunks = need[3];
+    level_hubs = units;
     if (units == 0 || (units <= work.hub_units && parts <= work.hub_parts && links <= work.hub_links &&
                        chunks <= work.hub_chunks))
         return;
@@ -949,6 +943,14 @@ void rmx_graph::stage_sweeps(Level &lv, bool allow_new, std::vector<double> &L, 
     int64_t n_active = lv.n;
     all_units(lv.n, work, stream);
     if (lv.n > 0) ensure_hub_table(lv);
+    if (fused_ok(lv)) {
+        if (!any_set(act) || opt.max_iter <= 0) return;
+        set_active(act);
+        run_fused(lv, mods, inst1, prior, allow_new, false, vthresh, sub_batches_for(lv.n));
+        RMX_CUDA(cudaMemcpyAsync(L.data(), inst1.L, sizeof(double) * K, cudaMemcpyDeviceToHost, stream));
+        RMX_CUDA(cudaStreamSynchronize(stream));
+        return;
+    }
     if (stage_graph_ok(lv)) {
         stage_sweeps_graph(lv, allow_new, L, act);
         return;
@@ -971,6 +973,26 @@ void rmx_graph::stage_sweeps(Level &lv, bool allow_new, std::vector<double> &L, 
             if (sweeping[k] && oldL[k] - L[k] >= 0 && (oldL[k] - L[k]) / kLn2 < opt.threshold) sweeping[k] = 0;
     }
     timers.end(lvt, stream);
+}
+
+// A stage runs as one cooperative launch on levels without hub units, never
+// with profiling events or per-sweep printing.
+bool rmx_graph::fused_ok(const Level &lv) const {
+    return level_hubs == 0 && !timers.on && opt.verbose < 2 && lv.n > 0;
+}
+
+// One stage as one launch (fused_stage), its sweeps and stamps counted on.
+void rmx_graph::run_fused(Level &lv, ModState &M, InstState &I, bool prior, bool allow_new, bool subtune,
+                          double vthresh, int ns) {
+    const FusedStage f{prior ? 1 : 0, allow_new ? 1 : 0, subtune ? 1 : 0, opt.max_iter, ns,    vthresh,
+                       opt.threshold, kLn2,              run_seed,         stamp,        sweep_no};
+    fused_stage(lv, M, I, work, f, stage_ctl, scratch, stream);
+    int64_t sweeps = 0;
+    RMX_CUDA(cudaMemcpyAsync(&sweeps, stage_ctl, sizeof sweeps, cudaMemcpyDeviceToHost, stream));
+    RMX_CUDA(cudaStreamSynchronize(stream));
+    sweep_no += (uint64_t)sweeps;
+    stamp += (uint32_t)(sweeps * ns);
+    prof.sweeps += sweeps;
 }
 
 // The stage loop runs as one captured graph once the handle has completed a
@@ -1220,12 +1242,14 @@ void rmx_graph::generate_sub_modules() {
         SweepArgs sa{0.0, 0};  // Network::move: best < 0, no empty module (Module.cpp:606, :667)
         timers.begin(kTimerLvSub, stream);
         const int nsg = sub_batches_for(N);
-        if (stage_graph_ok(sub_lv) && opt.max_iter > 0) {
+        const bool fused = fused_ok(sub_lv);
+        if (fused && opt.max_iter > 0) run_fused(sub_lv, submods, instsub, false, false, true, 0.0, nsg);
+        if (!fused && stage_graph_ok(sub_lv) && opt.max_iter > 0) {
             const StageGraphKey key{&sub_lv, &submods, &instsub, 0, 0, opt.max_iter, nsg, 0.0, opt.threshold,
                                     work.hub_gen, eval_tuning_generation(), scratch.mark()};
             loop_graph(key, N, [&](unsigned long long cond) { subtune_body(nsg, cond); });
         }
-        for (int iter = 0; iter < opt.max_iter && !stage_graph_ok(sub_lv); iter++) {
+        for (int iter = 0; iter < opt.max_iter && !fused && !stage_graph_ok(sub_lv); iter++) {
             all_units(N, work, stream);
             const uint32_t seed = mix_seed(run_seed, ++sweep_no);
             const int ns = sub_batches_for(N);

@@ -32,13 +32,15 @@ struct Level {
     int32_t *nnodes = nullptr;  // original nodes inside each unit
 };
 
-// A module's statistics and cached terms in one 64-byte record (two sectors
-// of one 128-byte line): what the move evaluation reads per candidate, so a
-// candidate costs one random line instead of one in each of two arrays.
+// What the move evaluation reads per candidate module, in one 64-byte record
+// (two sectors of one 128-byte line): its statistics in FP64 with what every
+// candidate derives from them (exit flow, alpha P + beta D), and its cached
+// terms. Written with the terms, so a candidate converts and combines nothing
+// that depends on the module alone.
 struct __align__(64) ModRec {
-    Stat4 s;
-    double2 t;
-    double2 pad;
+    double P, TW, em, g;  // flow, teleport weight, exit, alpha P + beta D
+    double2 t;            // {plogp(exit), plogp(exit + P)}
+    double D, pad;
 };
 
 struct ModState {
@@ -258,6 +260,18 @@ void free_modules(const ModState &M, SweepWork &W, Arena &ar, cudaStream_t s);
 // same choices. fitted: use the host bin sizes (see bucket_units).
 void sweep_subbatch(const Level &L, ModState &M, const InstState &I, SweepWork &W, const SweepArgs &a, int sb,
                     const uint32_t *sp, bool mark_active, bool fitted, cudaStream_t s, Timers *tm);
+// A whole stage of sweeps and its stop rule as one cooperative launch
+// (rmx_stage.cu), for levels without hub units. The level's units all start
+// active; I.active says which instances take part. subtune: the coarse-tune
+// sub-problems' stop rule. ctl (device): [0] the sweeps run.
+struct FusedStage {
+    int prior, allow_new, subtune, max_iter, nsub;
+    double vthresh, threshold, ln2;
+    uint32_t run_seed, stamp;     // stamp: of the last sub-batch so far
+    uint64_t sweep_no;            // sweeps so far
+};
+void fused_stage(const Level &lv, ModState &M, InstState &I, SweepWork &W, const FusedStage &f, int64_t *ctl, Arena &ar,
+                 cudaStream_t s);
 // Move evaluation only, for the parity hook (no commit).
 void evaluate_all(const Level &L, const ModState &M, const InstState &I, SweepWork &W, const uint8_t *allow_new,
                   double vthresh, Arena &ar, cudaStream_t s);

@@ -111,6 +111,7 @@ struct rmx_graph {
     rmx::Arena hub_arena, agg_arena;
     rmx::fx_t *agg_tab = nullptr;
     int64_t agg_cap = 0;
+    int64_t level_hubs = 0;  // hub units of the level ensure_hub_table last saw
 
     // ---- instances: 1 for a single graph; a batch is a disjoint union of
     // graph-attempt copies, node ranges inst_noff[k]..inst_noff[k+1]
@@ -188,6 +189,9 @@ struct rmx_graph {
     void stage_sweeps(rmx::Level &lv, bool allow_new, std::vector<double> &L, const std::vector<uint8_t> &act);
     void sweep_single(rmx::Level &lv, bool prior, bool allow_new, double vthresh, int64_t &n_active,
                       std::vector<double> &L);
+    bool fused_ok(const rmx::Level &lv) const;
+    void run_fused(rmx::Level &lv, rmx::ModState &M, rmx::InstState &I, bool prior, bool allow_new, bool subtune,
+                   double vthresh, int ns);
     bool stage_graph_ok(const rmx::Level &lv) const;
     void stage_sweeps_graph(rmx::Level &lv, bool allow_new, std::vector<double> &L, const std::vector<uint8_t> &act);
     void stage_body(rmx::Level &lv, bool allow_new, bool prior, double vthresh, int ns, unsigned long long cond);

@@ -25,122 +25,16 @@
 #include <stdexcept>
 #include <vector>
 
-#include "rmx_engine.cuh"
+#include "rmx_moves.cuh"
 
 // links each thread of a shared-table bin gathers ahead of its table inserts
 #ifndef RMX_EVAL_ILP
 #define RMX_EVAL_ILP 4
 #endif
-// the total-exit term of every candidate through log1p of a per-unit log (1) or a log each (0)
-#ifndef RMX_LOG1P
-#define RMX_LOG1P 1
-#endif
 
 namespace rmx {
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int32_t kEmpty = -1;
-constexpr int32_t kNewMod = -2;
-
-// ---------------------------------------------------------------- helpers
-
-__device__ __forceinline__ uint32_t mix32(uint32_t x) {
-    x ^= x >> 16;
-    x *= 0x7feb352dU;
-    x ^= x >> 15;
-    x *= 0x846ca68bU;
-    x ^= x >> 16;
-    return x;
-}
-
-__device__ __forceinline__ int tab_slot(int32_t key, int mask) { return (int)(mix32((uint32_t)key) & (uint32_t)mask); }
-
-__device__ __forceinline__ bool better(double d1, int32_t m1, double d2, int32_t m2) {
-    return d1 < d2 || (d1 == d2 && m1 < m2);
-}
-
-// Everything about the moving unit that every candidate needs. The terms of
-// the code-length change that depend only on the unit and its old module
-// (Module.cpp:1109-1112: sumAllExitPr, exit and stay of the old module before
-// and after) are folded into K once per unit.
-struct UnitCtx {
-    double pu, tu, eu, cu;  // flow, teleport weight, exit, tau*p + (1-tau)*d
-    double eA, nexA;        // old module exit before / after the unit leaves
-    double sum_exit;
-    double K;               // -plogp(se) - 2 (plogp(nexA) - plogp(eA)) + plogp(nexA + nPA) - plogp(eA + PA)
-    double S0, logS0, rS0;  // the new total exit without the target's change, its log and reciprocal
-    int32_t A;
-};
-
-// plogp of the new total exit flow S0 + dm, where dm = (new - old exit of the
-// target module) is tiny next to S0 for almost every candidate: then
-// log(S0 + dm) = log(S0) + log1p(dm / S0) with log(S0) computed once per unit
-// and log1p by its Mercator series through t^6 (|t| < 2^-10: truncation below
-// 2^-70 / 7 of the value, far under FP64 rounding); otherwise the direct log.
-__device__ __forceinline__ double plogp_total(const UnitCtx &c, double dm) {
-#if RMX_LOG1P
-    const double t = dm * c.rS0;
-    if (c.rS0 > 0.0 && fabs(t) < 0x1p-10) {
-        const double l1p = t * (1.0 - t * (0.5 - t * (1.0 / 3.0 - t * (0.25 - t * (0.2 - t * (1.0 / 6.0))))));
-        return (c.S0 + dm) * (c.logS0 + l1p);
-    }
-#endif
-    return plogp(c.S0 + dm);
-}
-
-// Change of moving the unit into module with statistics st, given the unit's
-// link flow to and from it (fixed point, out-links plus in-links, before the
-// 1-tau factor): d_all - 2 d_exit + d_stay of Module.cpp:1109-1115 with the
-// unit terms in K. The out- and in-flows (Module.cpp:1058, :1059) enter the
-// change only through their sum (the new exit, :1104), so the tables keep one
-// sum per module. t = the module's cached {plogp(exit), plogp(exit + P)}.
-__device__ __forceinline__ double candidate_delta(const UnitCtx &c, const ModRec &r, fx_t sfx) {
-    const Stat4 &st = r.s;
-    const double2 t = r.t;
-    const double P = from_fx(st.P), TW = from_fx(st.TW), D = from_fx(st.D), OUT = from_fx(st.OUT);
-    const double em = exit_flow(P, TW, D, OUT);
-    const double om_im = kBeta * from_fx(sfx) + c.cu * TW + (kAlpha * P + kBeta * D) * c.tu;  // :1058 + :1059
-    const double nexm = em + c.eu - om_im;                                                    // Module.cpp:1104
-    // new total exit sumAllExitPr + (nexA - eA) + (nexm - em), Module.cpp:1106
-    return plogp_total(c, nexm - em) + c.K - 2.0 * (plogp(nexm) - t.x) + (plogp(nexm + P + c.pu) - t.y);
-}
-
-// The empty-module option: exit e_u, no shared flow (Module.cpp:1072-1077).
-__device__ __forceinline__ double newmod_delta(const UnitCtx &c) {
-    const double nexm = c.eu;
-    return plogp_total(c, nexm) + c.K - 2.0 * plogp(nexm) + plogp(nexm + c.pu);
-}
-
-__device__ __forceinline__ UnitCtx make_ctx(const Stat4 &ua, const ModRec &mA, double sum_exit, int32_t A,
-                                            fx_t sA) {
-    const Stat4 &ma = mA.s;
-    const double2 tA = mA.t;
-    UnitCtx c;
-    c.pu = from_fx(ua.P);
-    c.tu = from_fx(ua.TW);
-    const double du = from_fx(ua.D);
-    c.eu = exit_flow(c.pu, c.tu, du, from_fx(ua.OUT));
-    c.cu = kAlpha * c.pu + kBeta * du;
-    const double PA = from_fx(ma.P), TWA = from_fx(ma.TW), DA = from_fx(ma.D);
-    c.eA = exit_flow(PA, TWA, DA, from_fx(ma.OUT));
-    // outFlow + inFlow to the old module (Module.cpp:1047, :1048), sA = their link flows' sum
-    const double outA_inA = kBeta * from_fx(sA) + c.cu * (TWA - c.tu) +
-                            (kAlpha * (PA - c.pu) + kBeta * (DA - du)) * c.tu;
-    c.nexA = c.eA - c.eu + outA_inA;  // :1084
-    c.sum_exit = sum_exit;
-    c.K = -plogp(sum_exit) - 2.0 * (plogp(c.nexA) - tA.x) + (plogp(c.nexA + (PA - c.pu)) - tA.y);
-    c.S0 = sum_exit + c.nexA - c.eA;
-#if RMX_LOG1P
-    const bool pos = c.S0 > 0.0;
-    c.logS0 = pos ? log(c.S0) : 0.0;
-    c.rS0 = pos ? 1.0 / c.S0 : 0.0;
-#else
-    c.logS0 = c.rS0 = 0.0;
-#endif
-    c.A = A;
-    return c;
-}
-
 struct EvalArgs {
     // level
     const int64_t *out_off, *in_off;
@@ -219,11 +113,6 @@ __device__ __forceinline__ void mark_neighbours(const EvalArgs &a, int32_t u, in
 // dense candidate list, and evaluate the candidates with all lanes.
 
 constexpr int kWarpMaxDeg = 128, kWarpCap = 256, kEvalWarps = 8;
-// degree bins: 8 / 16 / 32 lanes in registers, warp (shared table), block
-// (shared table), hub (global table)
-constexpr int kBins = 8;
-constexpr int kBinReg8 = 0, kBinReg16 = 1, kBinReg32 = 2, kBinWarp = 3, kBinMid = 4, kBinBlock = 5, kBinLarge = 6,
-              kBinHub = 7;
 // units of 129..512 links: four warps each (eight teams per SM), a 1024-slot table
 #ifndef RMX_MID_CAP
 #define RMX_MID_CAP 1024
@@ -942,7 +831,7 @@ __global__ void __launch_bounds__(kHubPT, RMX_HUB_MINB) k_hub_eval(EvalArgs a, H
         const int32_t u = a.list[h0 + j];
         const int64_t b0 = p.pstart[pidx], b1 = p.pstart[pidx + 1];
         const int32_t A = a.mod[u];
-        const UnitCtx c = make_ctx(a.attr[u], a.mrec[A], a.inst_sum_exit[a.uinst[u]], A, p.own[j]);
+        const UnitCtx c = make_ctx<true>(a.attr[u], a.mrec[A], a.inst_sum_exit[a.uinst[u]], A, p.own[j]);
         double best = 0.0;
         int32_t bm = INT_MAX;
         for (uint32_t R = 1;; R <<= 1) {  // R rounds; more only when a round overfills the table
@@ -1062,7 +951,7 @@ __global__ void k_hub_finish(EvalArgs a, HubPlan p) {
         }
         if (lane == 0) {
             const int32_t A = a.mod[u];
-            const UnitCtx c = make_ctx(a.attr[u], a.mrec[A], a.inst_sum_exit[a.uinst[u]], A,
+            const UnitCtx c = make_ctx<true>(a.attr[u], a.mrec[A], a.inst_sum_exit[a.uinst[u]], A,
                                        p.own[j]);
             p.act[j] = (uint8_t)finish_unit(a, u, c, best, bm);
             seen += unit_links(a, u);
@@ -1108,10 +997,6 @@ struct CommitArgs {
     // function of attempt seed, sweep and sub-batch) picks the free id a unit bids for
     const uint32_t *sp;
 };
-
-__device__ __forceinline__ unsigned long long claim_key(uint32_t stamp, int32_t u) {
-    return ((unsigned long long)stamp << 32) | (0xffffffffu - (uint32_t)u);
-}
 
 // Units proposing an empty module bid for a free id chosen by hash; the
 // smallest unit id wins each id (atomicMax on an inverted key), losers stay.
@@ -1276,21 +1161,6 @@ __global__ void __launch_bounds__(256) k_delta_block(DeltaArgs a) {
 }
 
 // ---------------------------------------------------------------- stats
-
-__device__ __forceinline__ double2 module_terms(const Stat4 &st) {
-    const double P = from_fx(st.P);
-    const double e = exit_flow(P, from_fx(st.TW), from_fx(st.D), from_fx(st.OUT));
-    return make_double2(plogp(e), plogp(e + P));
-}
-
-// A module's cached terms and its evaluation record.
-__device__ __forceinline__ void write_terms(const Stat4 *mstat, double2 *term, ModRec *rec, int32_t m) {
-    const Stat4 st = mstat[m];
-    const double2 t = module_terms(st);
-    term[m] = t;
-    rec[m].s = st;
-    rec[m].t = t;
-}
 
 __global__ void k_terms_all(int32_t cap, const Stat4 *mstat, double2 *term, ModRec *rec) {
     for (int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; m < cap; m += (int64_t)gridDim.x * blockDim.x)
@@ -1724,11 +1594,6 @@ void all_units(int32_t n, SweepWork &W, cudaStream_t s) {
     k_iota<<<blocks_for(n, 256, num_sms() * 32), 256, 0, s>>>(W.list, n, W.counters + kCntActive);
     RMX_LAUNCHED();
 }
-
-// Upper degree bounds of the warp, mid, block and large bins (run-time tuning).
-struct BinBounds {
-    int32_t warp, mid, block, large;
-};
 
 __global__ void k_bucket(const int32_t *list, const int64_t *n_active, const int64_t *out_off, const int64_t *in_off,
                          uint32_t seed, const uint32_t *seed_dev, int nsub, BinBounds bb, uint16_t *bucket) {
