@@ -448,7 +448,7 @@ void rmx_graph::adjoint(const int32_t *part_host, double tau, double *L_out, dou
     RMX_CUDA(cudaMemcpyAsync(part, part_host, sizeof(int32_t) * N, cudaMemcpyHostToDevice, stream));
     RMX_CUDA(cudaMemsetAsync(mst, 0, sizeof(Stat4) * N, stream));
     RMX_CUDA(cudaMemsetAsync(s0, 0, sizeof(fx_t), stream));
-    power_iteration(N, in_off, in_src, in_w, tw, dangling, pa, A, stream, spmv_vec, tau);
+    power_iteration(N, E, in_off, in_src, in_w, tw, dangling, pa, A, stream, spmv_vec, tau);
     k_adj_rows<<<blocks_for((int64_t)N * 32, 256, num_sms() * 32), 256, 0, stream>>>(
         N, out_off, out_dst, out_w0, part, pa, tw, dangling, rowsum, cross, mst, s0);
     RMX_LAUNCHED();

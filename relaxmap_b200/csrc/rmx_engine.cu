@@ -766,7 +766,7 @@ void rmx_graph::initiate() {
     timers.end(kTimerOther, stream);
     timers.begin(kTimerSpmv, stream);
     if (K == 1)
-        power_iters = power_iteration(N, in_off, in_src, in_w, tw, dangling, p, scratch, stream, spmv_vec);
+        power_iters = power_iteration(N, E, in_off, in_src, in_w, tw, dangling, p, scratch, stream, spmv_vec);
     else
         power_iters = union_flows();
     timers.end(kTimerSpmv, stream);

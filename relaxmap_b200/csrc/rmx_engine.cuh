@@ -86,11 +86,11 @@ struct FlowOut {
     int iters = 0;
 };
 // alpha: teleportation probability (the reference's 0.15 unless a caller varies it).
-int power_iteration(int32_t n, const int64_t *in_off, const int32_t *in_src, const double *in_w, const double *tw,
+int power_iteration(int32_t n, int64_t m, const int64_t *in_off, const int32_t *in_src, const double *in_w, const double *tw,
                     const uint8_t *dangling, double *p, Arena &ar, cudaStream_t s, int vec, double alpha = kAlpha);
 // The same solve writing into caller-provided scratch (y[n], parts[3*max_blocks],
 // iters on the device); asynchronous, allocates nothing.
-void power_iteration_into(int32_t n, const int64_t *in_off, const int32_t *in_src, const double *in_w,
+void power_iteration_into(int32_t n, int64_t m, const int64_t *in_off, const int32_t *in_src, const double *in_w,
                           const double *tw, const uint8_t *dangling, double *p, double *y, double *parts,
                           int max_blocks, int *iters, cudaStream_t s, int vec);
 // The stationary flow of every component of a disjoint union: one block per

@@ -16,6 +16,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <mutex>
 #include <vector>
 
 #include "rmx_engine.cuh"
@@ -247,27 +248,32 @@ __device__ __forceinline__ double block_sum(double v, double *sh) {
     return t;  // valid in thread 0
 }
 
-// Sum of nb per-block partials in one fixed order; every block and thread gets
-// the identical value.
-__device__ __forceinline__ double sum_parts(const double *parts, int nb, double *sh) {
-    if (threadIdx.x < 32) {
-        double v = 0.0;
-        for (int i = threadIdx.x; i < nb; i += 32) v += __ldcg(parts + i);
+// Sum of nb per-block partials in one fixed order (lane-strided, then a
+// butterfly), by the calling warp; loads run eight ahead of the additions.
+__device__ __forceinline__ double warp_sum_parts(const double *parts, int nb, int lane) {
+    double v = 0.0;
+    for (int i0 = lane; i0 < nb; i0 += 256) {
+        double t[8];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-        if (threadIdx.x == 0) sh[0] = v;
+        for (int k = 0; k < 8; k++) t[k] = i0 + 32 * k < nb ? __ldcg(parts + i0 + 32 * k) : 0.0;
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (i0 + 32 * k < nb) v += t[k];
     }
-    __syncthreads();
-    double r = sh[0];
-    __syncthreads();
-    return r;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+    return v;
 }
 
 constexpr int kPowT = 256;
-// resident blocks per SM the power iteration is compiled for (and launched with)
+// The iteration's sums (total flow, L1 change, dangling mass) are formed per
+// "virtual" block of kPowT threads of a fixed grid, kPowGrid such blocks per
+// SM, and added in block order: their rounding, which the 1e-15 stop rule sits
+// on, does not depend on how many blocks are launched or in which form.
 #ifndef RMX_POW_MINB
 #define RMX_POW_MINB 6
 #endif
+constexpr int kPowGrid = 6, kPowWarps = kPowT / 32;
 
 // Rows of more than heavy_deg in-links (in-degree hubs) are not left to one
 // lane group: their links come in chunks of kPowChunk, a warp per chunk, and
@@ -280,6 +286,7 @@ struct PowSplit {
     const int64_t *chunk_beg = nullptr, *chunk_end = nullptr;  // link range of every chunk
     int64_t n_chunks = 0;
     double *cpart = nullptr;             // partial pull of every chunk
+    double *ls = nullptr;                // per thread of the virtual grid: its light rows' sum
     int64_t heavy_deg = INT64_MAX;
 };
 
@@ -299,103 +306,133 @@ __global__ void __launch_bounds__(kPowT, RMX_POW_MINB) k_power(const int64_t *__
                                                  const double *__restrict__ in_w, const double *__restrict__ tw,
                                                  const uint8_t *__restrict__ dang, int32_t n, double *x, double *y,
                                                  double *parts, int *iters_out, double alpha, PowSplit sp,
-                                                 PowGather pg) {
+                                                 PowGather pg, int nb) {
     cg::grid_group grid = cg::this_grid();
     __shared__ double sh[32];
-    const int nb = gridDim.x;
+    __shared__ double shared_sum[2];
     double *Sp = parts, *Dp = parts + nb, *Ep = parts + 2 * nb;
-    const int64_t gtid = (int64_t)blockIdx.x * kPowT + threadIdx.x, gthreads = (int64_t)nb * kPowT;
+    const int64_t gthreads = (int64_t)nb * kPowT, nwarps = gthreads >> 5;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane / VEC, lv = lane % VEC;
+    constexpr int RPW = 32 / VEC;  // rows per warp step
+    const double beta = 1.0 - alpha;  // 1.0 - 0.15 is kBeta exactly
 
     // the link arrays are streamed with the evict-first hint so that the
     // gathered vector stays in L2 between iterations
-    const double *xg = pg.gsrc ? pg.xc : x;        // the vector the pull gathers from
+    const double *xg = pg.gsrc ? pg.xc : x;          // the vector the pull gathers from
     const int32_t *gs = pg.gsrc ? pg.gsrc : in_src;  // and the links' places in it
-    double dl = 0.0;
     const double x0 = 1.0 / n;
-    for (int64_t i = gtid; i < n; i += gthreads) {
-        x[i] = x0;
-        if (pg.gsrc && pg.rank[i] >= 0) pg.xc[pg.rank[i]] = x0;
-        if (dang[i]) dl += x0;
+    for (int vb = blockIdx.x; vb < nb; vb += gridDim.x) {
+        double dl = 0.0;
+        for (int64_t i = (int64_t)vb * kPowT + threadIdx.x; i < n; i += gthreads) {
+            x[i] = x0;
+            if (pg.gsrc && pg.rank[i] >= 0) pg.xc[pg.rank[i]] = x0;
+            if (dang[i]) dl += x0;
+        }
+        dl = block_sum<kPowT>(dl, sh);
+        if (threadIdx.x == 0) Dp[vb] = dl;
     }
-    dl = block_sum<kPowT>(dl, sh);
-    if (threadIdx.x == 0) Dp[blockIdx.x] = dl;
     grid.sync();
-
-    constexpr int RPW = 32 / VEC;  // rows per warp per step
-    const int lane = threadIdx.x & 31, sub = lane / VEC, lv = lane % VEC;
-    const int64_t gwarp = gtid >> 5, nwarps = gthreads >> 5;
+    if (warp == 0) {
+        const double v = warp_sum_parts(Dp, nb, lane);
+        if (lane == 0) shared_sum[1] = v;
+    }
+    __syncthreads();
     int iter = 0;
     for (;;) {
-        const double D = sum_parts(Dp, nb, sh);
-        const double beta = 1.0 - alpha;  // 1.0 - 0.15 is kBeta exactly
+        const double D = shared_sum[1];
         const double coef = alpha + beta * D;
-        double ls = 0.0;
-        for (int64_t base = gwarp * RPW; base < n; base += nwarps * RPW) {
-            const int64_t r = base + sub;
-            double acc = 0.0;
-            bool mine = r < n;
-            if (mine) {
-                const int64_t b = in_off[r], e = in_off[r + 1];
-                mine = e - b <= sp.heavy_deg;
-                if (mine)
-                    for (int64_t k = b + lv; k < e; k += VEC) acc += beta * __ldcs(in_w + k) * __ldcg(xg + __ldcs(gs + k));
-            }
-#pragma unroll
-            for (int o = VEC / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(kFull, acc, o);
-            if (mine && lv == 0) {
-                const double v = coef * tw[r] + acc;
-                y[r] = v;
-                ls += v;
-            }
-        }
-        if (sp.n_rows > 0) {  // the same branch in every block
-            for (int64_t c = gwarp; c < sp.n_chunks; c += nwarps) {
+        for (int vb = blockIdx.x; vb < nb; vb += gridDim.x) {
+            double ls = 0.0;
+            const int64_t gwarp = (int64_t)vb * kPowWarps + warp;
+            for (int64_t base = gwarp * RPW; base < n; base += nwarps * RPW) {
+                const int64_t r = base + sub;
                 double acc = 0.0;
-                for (int64_t k = sp.chunk_beg[c] + lane; k < sp.chunk_end[c]; k += 32)
-                    acc += beta * __ldcs(in_w + k) * __ldcg(xg + __ldcs(gs + k));
+                bool mine = r < n;
+                if (mine) {
+                    const int64_t b = in_off[r], e = in_off[r + 1];
+                    mine = e - b <= sp.heavy_deg;
+                    if (mine)
+                        for (int64_t k = b + lv; k < e; k += VEC)
+                            acc += beta * __ldcs(in_w + k) * __ldcg(xg + __ldcs(gs + k));
+                }
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(kFull, acc, o);
-                if (lane == 0) sp.cpart[c] = acc;
-            }
-            grid.sync();
-            for (int64_t h = gwarp; h < sp.n_rows; h += nwarps) {
-                const int32_t r = sp.rows[h];
-                double acc = 0.0;
-                for (int64_t c = sp.row_chunk[h] + lane; c < sp.row_chunk[h + 1]; c += 32) acc += __ldcg(sp.cpart + c);
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(kFull, acc, o);
-                if (lane == 0) {
+                for (int o = VEC / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(kFull, acc, o);
+                if (mine && lv == 0) {
                     const double v = coef * tw[r] + acc;
                     y[r] = v;
                     ls += v;
                 }
             }
+            if (sp.n_rows > 0) {  // the same branch in every block
+                for (int64_t c = gwarp; c < sp.n_chunks; c += nwarps) {
+                    double acc = 0.0;
+                    for (int64_t k = sp.chunk_beg[c] + lane; k < sp.chunk_end[c]; k += 32)
+                        acc += beta * __ldcs(in_w + k) * __ldcg(xg + __ldcs(gs + k));
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(kFull, acc, o);
+                    if (lane == 0) sp.cpart[c] = acc;
+                }
+                sp.ls[(int64_t)vb * kPowT + threadIdx.x] = ls;  // until the chunks are all there
+            } else {
+                ls = block_sum<kPowT>(ls, sh);
+                if (threadIdx.x == 0) Sp[vb] = ls;
+            }
         }
-        ls = block_sum<kPowT>(ls, sh);
-        if (threadIdx.x == 0) Sp[blockIdx.x] = ls;
+        if (sp.n_rows > 0) {
+            grid.sync();
+            for (int vb = blockIdx.x; vb < nb; vb += gridDim.x) {
+                double ls = sp.ls[(int64_t)vb * kPowT + threadIdx.x];
+                for (int64_t h = (int64_t)vb * kPowWarps + warp; h < sp.n_rows; h += nwarps) {
+                    const int32_t r = sp.rows[h];
+                    double acc = 0.0;
+                    for (int64_t c = sp.row_chunk[h] + lane; c < sp.row_chunk[h + 1]; c += 32)
+                        acc += __ldcg(sp.cpart + c);
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(kFull, acc, o);
+                    if (lane == 0) {
+                        const double v = coef * tw[r] + acc;
+                        y[r] = v;
+                        ls += v;
+                    }
+                }
+                ls = block_sum<kPowT>(ls, sh);
+                if (threadIdx.x == 0) Sp[vb] = ls;
+            }
+        }
         grid.sync();
-        const double S = sum_parts(Sp, nb, sh);
-        double el = 0.0;
-        dl = 0.0;
-        for (int64_t i = gtid; i < n; i += gthreads) {
-            const double xn = __ldcg(y + i) / S;
-            el += fabs(xn - x[i]);
-            x[i] = xn;
-            if (pg.gsrc && pg.rank[i] >= 0) pg.xc[pg.rank[i]] = xn;
-            if (dang[i]) dl += xn;
+        if (warp == 0) {
+            const double v = warp_sum_parts(Sp, nb, lane);
+            if (lane == 0) shared_sum[0] = v;
         }
-        el = block_sum<kPowT>(el, sh);
-        dl = block_sum<kPowT>(dl, sh);
-        if (threadIdx.x == 0) {
-            Ep[blockIdx.x] = el;
-            Dp[blockIdx.x] = dl;
+        __syncthreads();
+        const double S = shared_sum[0];
+        for (int vb = blockIdx.x; vb < nb; vb += gridDim.x) {
+            double el = 0.0, dl = 0.0;
+            for (int64_t i = (int64_t)vb * kPowT + threadIdx.x; i < n; i += gthreads) {
+                const double xn = __ldcg(y + i) / S;
+                el += fabs(xn - x[i]);
+                x[i] = xn;
+                if (pg.gsrc && pg.rank[i] >= 0) pg.xc[pg.rank[i]] = xn;
+                if (dang[i]) dl += xn;
+            }
+            el = block_sum<kPowT>(el, sh);
+            dl = block_sum<kPowT>(dl, sh);
+            if (threadIdx.x == 0) {
+                Ep[vb] = el;
+                Dp[vb] = dl;
+            }
         }
         grid.sync();
-        const double diff = sum_parts(Ep, nb, sh);
+        if (warp < 2) {
+            const double v = warp_sum_parts(warp ? Dp : Ep, nb, lane);
+            if (lane == 0) shared_sum[warp] = v;
+        }
+        __syncthreads();
+        const double diff = shared_sum[0];
         iter++;
         if (iter >= 200 || (diff <= 1.0e-15 && iter >= 50)) break;  // Module.cpp:460
     }
-    if (gtid == 0) *iters_out = iter;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *iters_out = iter;
 }
 
 __global__ void k_pow_heavy_flags(int32_t n, const int64_t *in_off, int64_t heavy_deg, uint8_t *flag) {
@@ -510,28 +547,270 @@ static PowGather gather_copy(int32_t n, const int64_t *in_off, const int32_t *in
     return pg;
 }
 
+// ------------------------------------------------ small graphs: one cluster
+
+// The same iteration for small graphs by one thread-block cluster: the flow
+// vector in every block's shared memory (a new value is stored to all of
+// them), the partial sums too, and the cluster's hardware barrier (0.27 us)
+// where k_power has a grid barrier (1.25 us). A virtual block of k_power is 256
+// threads of a block here, with the same rows, lanes and order of additions, so
+// the result is the same bit for bit. Bound by two barriers and two chains of
+// dependent reductions per iteration. 50 iterations, 1003 nodes: 378 us through
+// k_power, 238 us here; 3001 nodes: 397 and 290 us. Rows of more than heavy_deg
+// links are left to k_power (*iters_out = -1, nothing computed).
+constexpr int kClT = 1024, kClGroups = kClT / kPowT, kClMaxSize = 16;
+// Largest graphs: every virtual warp has one step of rows, and a block has at
+// most 8 to 16 virtual blocks; the cluster's 16 SMs then take as long per
+// iteration as the whole grid (6003 nodes, 188 virtual blocks: 470 us here, 447
+// through k_power).
+constexpr int32_t kClMaxNodes = 8192, kClMaxBlocks = 128;
+constexpr int64_t kClMaxLinks = 1 << 17;
+
+__device__ __forceinline__ uint32_t cl_addr(const void *p, unsigned rank) {  // p's copy in block `rank` of the cluster
+    uint32_t a = (uint32_t)__cvta_generic_to_shared(p), r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cl_store(const void *p, unsigned rank, double v) {
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(cl_addr(p, rank)), "d"(v) : "memory");
+}
+__device__ __forceinline__ void cl_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// warp_sum_parts over shared memory.
+__device__ __forceinline__ double cl_sum_parts(const double *parts, int nb, int lane) {
+    double v = 0.0;
+#pragma unroll 4
+    for (int i = lane; i < nb; i += 32) v += parts[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+    return v;
+}
+
 template <int VEC>
-static int launch_power(int32_t n, const int64_t *in_off, const int32_t *in_src, const double *in_w, const double *tw,
-                        const uint8_t *dangling, double *p, Arena &ar, cudaStream_t s, double alpha) {
-    int dev = 0, per_sm = 0, coop = 0;
+__global__ void __launch_bounds__(kClT, 1) k_power_cluster(const int64_t *__restrict__ in_off,
+                                                           const int32_t *__restrict__ in_src,
+                                                           const double *__restrict__ in_w,
+                                                           const double *__restrict__ tw,
+                                                           const uint8_t *__restrict__ dang, int32_t n, double *p,
+                                                           int *iters_out, double alpha, int nb, int64_t heavy_deg) {
+    extern __shared__ __align__(16) double cl_smem[];
+    double *const x = cl_smem, *const y = x + n;  // y: this block's elements, by virtual block
+    unsigned C, rank;
+    asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(C));
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    const int nbe = (n + kPowT - 1) / kPowT;  // virtual blocks with an element (one per thread)
+    const int ey = (nbe + (int)C - 1) / (int)C * kPowT;
+    double *const Sp = y + ey, *const Ep = Sp + nb, *const Dp = Ep + nbe;
+    constexpr int kMaxOwn = kClMaxBlocks / 8;  // virtual blocks of one block, of at least eight in the cluster
+    __shared__ double sh[2][kMaxOwn][kPowWarps];
+    __shared__ int any_heavy;
+    const int t = threadIdx.x & (kPowT - 1), grp = threadIdx.x / kPowT, w = t >> 5, lane = threadIdx.x & 31;
+    const int sub = lane / VEC, lv = lane % VEC, bw = threadIdx.x >> 5;
+    constexpr int RPW = 32 / VEC;
+    const double beta = 1.0 - alpha;
+    // Virtual block vb is number vb / C of block vb % C; group g takes numbers g, g + 4, ...
+    const int own = ((int)nb - (int)rank + (int)C - 1) / (int)C, owne = (nbe - (int)rank + (int)C - 1) / (int)C;
+    auto warp_total = [&](double v) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+        return v;
+    };
+    // The sums of cnt of this block's virtual blocks, each from its eight warps' sums in
+    // block_sum's order, stored to every block: warp c to block c.
+    auto send = [&](const double (*q)[kPowWarps], int cnt, double *parts) {
+        for (unsigned c = bw; c < C; c += kClT / 32)
+            for (int k = lane; k < cnt; k += 32)
+                cl_store(parts + k * (int)C + (int)rank, c,
+                         ((q[k][0] + q[k][4]) + (q[k][2] + q[k][6])) + ((q[k][1] + q[k][5]) + (q[k][3] + q[k][7])));
+    };
+    if (threadIdx.x == 0) any_heavy = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += kClT)
+        if (in_off[i + 1] - in_off[i] > heavy_deg) any_heavy = 1;
+    __syncthreads();
+    if (any_heavy) {  // the same in every block; no other block's memory has been touched
+        if (rank == 0 && threadIdx.x == 0) *iters_out = -1;
+        return;
+    }
+    cl_sync();  // the blocks have all started before one stores to another's memory
+    const double x0 = 1.0 / n;
+    for (int i = threadIdx.x; i < n; i += kClT) x[i] = x0;
+    for (int k = grp; k < owne; k += kClGroups) {
+        const int i = (k * (int)C + (int)rank) * kPowT + t;
+        const double s = warp_total(i < n && dang[i] ? x0 : 0.0);
+        if (lane == 0) sh[1][k][w] = s;
+    }
+    __syncthreads();
+    send(sh[1], owne, Dp);
+    cl_sync();
+    double D = cl_sum_parts(Dp, nbe, lane);
+    int iter = 0;
+    for (;;) {
+        const double coef = alpha + beta * D;
+#pragma unroll 2
+        for (int k = grp; k < own; k += kClGroups) {
+            const int r = ((k * (int)C + (int)rank) * kPowWarps + w) * RPW + sub;
+            double acc = 0.0, ls = 0.0;
+            if (r < n) {
+                const int e = (int)in_off[r + 1];
+#pragma unroll 4
+                for (int j = (int)in_off[r] + lv; j < e; j += VEC) acc += beta * in_w[j] * x[in_src[j]];
+            }
+#pragma unroll
+            for (int o = VEC / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(kFull, acc, o);
+            if (r < n && lv == 0) {
+                const double v = coef * tw[r] + acc;
+                const int ve = r / kPowT;  // the element's virtual block, held by block ve % C
+                cl_store(y + ve / (int)C * kPowT + r % kPowT, (unsigned)(ve % (int)C), v);
+                ls = v;
+            }
+            ls = warp_total(ls);
+            if (lane == 0) sh[0][k][w] = ls;
+        }
+        __syncthreads();
+        send(sh[0], own, Sp);
+        cl_sync();
+        const double S = cl_sum_parts(Sp, nb, lane);
+        for (int k = grp; k < owne; k += kClGroups) {
+            const int i = (k * (int)C + (int)rank) * kPowT + t;
+            double el = 0.0, dl = 0.0;
+            if (i < n) {
+                const double xn = y[k * kPowT + t] / S;
+                el = fabs(xn - x[i]);
+                if (dang[i]) dl = xn;
+                for (unsigned c = 0; c < C; c++) cl_store(x + i, c, xn);
+            }
+            el = warp_total(el);
+            dl = warp_total(dl);
+            if (lane == 0) {
+                sh[0][k][w] = el;
+                sh[1][k][w] = dl;
+            }
+        }
+        __syncthreads();
+        send(sh[0], owne, Ep);
+        send(sh[1], owne, Dp);
+        cl_sync();
+        const double diff = cl_sum_parts(Ep, nbe, lane);
+        D = cl_sum_parts(Dp, nbe, lane);
+        iter++;
+        if (iter >= 200 || (diff <= 1.0e-15 && iter >= 50)) break;
+    }
+    for (int i = (int)rank * kClT + threadIdx.x; i < n; i += (int)C * kClT) p[i] = x[i];
+    if (rank == 0 && threadIdx.x == 0) *iters_out = iter;
+}
+
+// The virtual grid's blocks for n rows.
+static int power_blocks(int32_t n, int vec, int max_nb) {
+    return (int)std::min<int64_t>(max_nb, std::max<int64_t>(1, ((int64_t)n * vec + kPowT - 1) / kPowT));
+}
+
+// Blocks of k_power launched for nb virtual blocks: all of them on large
+// graphs (six per SM: the pull wants every warp it can have); below 2^17 rows
+// half as many, each taking two (the barriers and the partial sums' readers
+// cost less: 30,001 nodes 828 -> 739 us for 50 iterations).
+template <int VEC>
+static int power_launch_grid(int32_t n, int nb) {
+    static std::mutex mu;
+    static std::vector<int> resident;  // per device
+    int dev = 0;
     RMX_CUDA(cudaGetDevice(&dev));
-    RMX_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-    if (!coop) throw CudaError(cudaErrorNotSupported, "cooperative launch not supported");
-    RMX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_power<VEC>, kPowT, 0));
-    int nb = std::max(1, std::min(per_sm, RMX_POW_MINB)) * num_sms();
-    nb = (int)std::min<int64_t>(nb, std::max<int64_t>(1, ((int64_t)n * VEC + kPowT - 1) / kPowT));
+    std::lock_guard<std::mutex> lk(mu);
+    if ((int)resident.size() <= dev) resident.resize(dev + 1, 0);
+    if (resident[dev] == 0) {
+        int coop = 0;
+        RMX_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+        if (!coop) throw CudaError(cudaErrorNotSupported, "cooperative launch not supported");
+        RMX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident[dev], k_power<VEC>, kPowT, 0));
+    }
+    if (resident[dev] < 1) throw CudaError(cudaErrorLaunchOutOfResources, "power iteration does not fit an SM");
+    const int res = std::min(resident[dev], n < (1 << 17) ? kPowGrid / 2 : kPowGrid) * num_sms();
+    const int turns = (nb + res - 1) / res;
+    return (nb + turns - 1) / turns;
+}
+
+// Runs the cluster form if the graph is small enough (false: it is not).
+// *iters (device) is -1 if a row is heavy; then nothing was computed.
+template <int VEC>
+static bool launch_power_cluster(int32_t n, int64_t m, const int64_t *in_off, const int32_t *in_src, const double *in_w,
+                                 const double *tw, const uint8_t *dangling, double *p, int *iters, double alpha,
+                                 int nb, int64_t heavy_deg, cudaStream_t s) {
+    if (n > kClMaxNodes || m > kClMaxLinks || nb > kClMaxBlocks || (int64_t)n * VEC > (int64_t)nb * kPowT) return false;
+    const int nbe = (n + kPowT - 1) / kPowT;
+    auto smem_for = [&](int C) {
+        return sizeof(double) * ((size_t)n + (size_t)((nbe + C - 1) / C) * kPowT + nb + 2 * (size_t)nbe);
+    };
+    static std::mutex mu;
+    static std::vector<int> size;  // per device: cluster size (0 not yet asked)
+    int dev = 0, C = 0;
+    RMX_CUDA(cudaGetDevice(&dev));
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    cfg.blockDim = dim3(kClT);
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        if ((int)size.size() <= dev) size.resize(dev + 1, 0);
+        if (size[dev] == 0) {
+            const size_t most = sizeof(double) * ((size_t)kClMaxNodes + kClMaxNodes / 8 + 3 * 1024);  // smem_for's largest
+            RMX_CUDA(cudaFuncSetAttribute(k_power_cluster<VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+            RMX_CUDA(cudaFuncSetAttribute(k_power_cluster<VEC>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            for (int c = kClMaxSize; c >= 1 && size[dev] == 0; c /= 2) {  // 16 blocks where a GPC has room for them
+                at[0].val.clusterDim.x = c;
+                cfg.gridDim = dim3(c);
+                cfg.dynamicSmemBytes = most;
+                int most_clusters = 0;
+                if (cudaOccupancyMaxActiveClusters(&most_clusters, k_power_cluster<VEC>, &cfg) == cudaSuccess &&
+                    most_clusters > 0)
+                    size[dev] = c;
+            }
+            (void)cudaGetLastError();
+            if (size[dev] == 0) size[dev] = -1;
+        }
+        C = size[dev];
+    }
+    if (C < 8) return false;
+    at[0].val.clusterDim.x = C;
+    cfg.gridDim = dim3(C);
+    cfg.dynamicSmemBytes = smem_for(C);
+    RMX_CUDA(cudaLaunchKernelEx(&cfg, k_power_cluster<VEC>, in_off, in_src, in_w, tw, dangling, n, p, iters, alpha, nb,
+                                heavy_deg));
+    RMX_LAUNCHED();
+    return true;
+}
+
+template <int VEC>
+static int launch_power(int32_t n, int64_t m, const int64_t *in_off, const int32_t *in_src, const double *in_w,
+                        const double *tw, const uint8_t *dangling, double *p, Arena &ar, cudaStream_t s, double alpha) {
+    int nb = power_blocks(n, VEC, kPowGrid * num_sms());
     size_t mk = ar.mark();
+    int *iters = ar.alloc<int>(1);
+    int h = 0;
+    if (launch_power_cluster<VEC>(n, m, in_off, in_src, in_w, tw, dangling, p, iters, alpha, nb, 64 * VEC, s)) {
+        RMX_CUDA(cudaMemcpyAsync(&h, iters, sizeof(int), cudaMemcpyDeviceToHost, s));
+        RMX_CUDA(cudaStreamSynchronize(s));
+        if (h >= 0) {
+            ar.release(mk);
+            return h;
+        }
+    }
     double *y = ar.alloc<double>(std::max(n, 1));
     double *parts = ar.alloc<double>(3 * nb);
-    int *iters = ar.alloc<int>(1);
     PowSplit sp = heavy_split(n, in_off, 64 * VEC, ar, s);
     PowGather pg = gather_copy(n, in_off, in_src, ar, s);
+    if (sp.n_rows > 0) sp.ls = ar.alloc<double>((size_t)nb * kPowT);
     void *args[] = {(void *)&in_off, (void *)&in_src, (void *)&in_w,  (void *)&tw,    (void *)&dangling, (void *)&n,
                     (void *)&p,      (void *)&y,      (void *)&parts, (void *)&iters, (void *)&alpha,    (void *)&sp,
-                    (void *)&pg};
-    RMX_CUDA(cudaLaunchCooperativeKernel((void *)k_power<VEC>, dim3(nb), dim3(kPowT), args, 0, s));
+                    (void *)&pg,     (void *)&nb};
+    RMX_CUDA(cudaLaunchCooperativeKernel((void *)k_power<VEC>, dim3(power_launch_grid<VEC>(n, nb)), dim3(kPowT), args, 0,
+                                         s));
     RMX_LAUNCHED();
-    int h = 0;
     RMX_CUDA(cudaMemcpyAsync(&h, iters, sizeof(int), cudaMemcpyDeviceToHost, s));
     RMX_CUDA(cudaStreamSynchronize(s));
     ar.release(mk);
@@ -541,41 +820,36 @@ static int launch_power(int32_t n, const int64_t *in_off, const int32_t *in_src,
 // Launch of the same solve into caller-provided scratch: y[n], parts[3 * max_blocks],
 // *iters; nothing is allocated and nothing waits on the stream.
 template <int VEC>
-static void launch_power_into(int32_t n, const int64_t *in_off, const int32_t *in_src, const double *in_w,
+static void launch_power_into(int32_t n, int64_t m, const int64_t *in_off, const int32_t *in_src, const double *in_w,
                               const double *tw, const uint8_t *dangling, double *p, double *y, double *parts,
                               int max_blocks, int *iters, cudaStream_t s) {
-    int dev = 0, per_sm = 0, coop = 0;
-    RMX_CUDA(cudaGetDevice(&dev));
-    RMX_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-    if (!coop) throw CudaError(cudaErrorNotSupported, "cooperative launch not supported on this device");
-    RMX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_power<VEC>, kPowT, 0));
-    int nb = std::max(1, std::min(per_sm, RMX_POW_MINB)) * num_sms();
-    nb = (int)std::min<int64_t>(nb, std::max<int64_t>(1, ((int64_t)n * VEC + kPowT - 1) / kPowT));
-    nb = std::min(nb, max_blocks);
+    int nb = power_blocks(n, VEC, std::min(kPowGrid * num_sms(), max_blocks));
     double alpha = kAlpha;
     // No chunked rows: in-degree hubs are pulled in one pass by their own
     // lanes (nothing beyond the caller's scratch), so on graphs with such
     // hubs the sums round differently from power_iteration's. No gathered copy.
+    if (launch_power_cluster<VEC>(n, m, in_off, in_src, in_w, tw, dangling, p, iters, alpha, nb, INT64_MAX, s)) return;
     PowSplit sp;
     PowGather pg;
     void *args[] = {(void *)&in_off, (void *)&in_src, (void *)&in_w,  (void *)&tw,    (void *)&dangling, (void *)&n,
                     (void *)&p,      (void *)&y,      (void *)&parts, (void *)&iters, (void *)&alpha,    (void *)&sp,
-                    (void *)&pg};
-    RMX_CUDA(cudaLaunchCooperativeKernel((void *)k_power<VEC>, dim3(nb), dim3(kPowT), args, 0, s));
+                    (void *)&pg,     (void *)&nb};
+    RMX_CUDA(cudaLaunchCooperativeKernel((void *)k_power<VEC>, dim3(power_launch_grid<VEC>(n, nb)), dim3(kPowT), args, 0,
+                                         s));
     RMX_LAUNCHED();
 }
 
-void power_iteration_into(int32_t n, const int64_t *in_off, const int32_t *in_src, const double *in_w,
+void power_iteration_into(int32_t n, int64_t m, const int64_t *in_off, const int32_t *in_src, const double *in_w,
                           const double *tw, const uint8_t *dangling, double *p, double *y, double *parts,
                           int max_blocks, int *iters, cudaStream_t s, int vec) {
     if (n <= 0) return;
     switch (vec) {
-        case 4: return launch_power_into<4>(n, in_off, in_src, in_w, tw, dangling, p, y, parts, max_blocks, iters, s);
-        case 8: return launch_power_into<8>(n, in_off, in_src, in_w, tw, dangling, p, y, parts, max_blocks, iters, s);
+        case 4: return launch_power_into<4>(n, m, in_off, in_src, in_w, tw, dangling, p, y, parts, max_blocks, iters, s);
+        case 8: return launch_power_into<8>(n, m, in_off, in_src, in_w, tw, dangling, p, y, parts, max_blocks, iters, s);
         case 16:
-            return launch_power_into<16>(n, in_off, in_src, in_w, tw, dangling, p, y, parts, max_blocks, iters, s);
+            return launch_power_into<16>(n, m, in_off, in_src, in_w, tw, dangling, p, y, parts, max_blocks, iters, s);
         default:
-            return launch_power_into<32>(n, in_off, in_src, in_w, tw, dangling, p, y, parts, max_blocks, iters, s);
+            return launch_power_into<32>(n, m, in_off, in_src, in_w, tw, dangling, p, y, parts, max_blocks, iters, s);
     }
 }
 
@@ -702,14 +976,14 @@ int spmv_width(double mean_in_degree) {
     return mean_in_degree <= 16 ? 4 : (mean_in_degree <= 24 ? 8 : (mean_in_degree <= 48 ? 16 : 32));
 }
 
-int power_iteration(int32_t n, const int64_t *in_off, const int32_t *in_src, const double *in_w, const double *tw,
+int power_iteration(int32_t n, int64_t m, const int64_t *in_off, const int32_t *in_src, const double *in_w, const double *tw,
                     const uint8_t *dangling, double *p, Arena &ar, cudaStream_t s, int vec, double alpha) {
     if (n <= 0) return 0;
     switch (vec) {
-        case 4: return launch_power<4>(n, in_off, in_src, in_w, tw, dangling, p, ar, s, alpha);
-        case 8: return launch_power<8>(n, in_off, in_src, in_w, tw, dangling, p, ar, s, alpha);
-        case 16: return launch_power<16>(n, in_off, in_src, in_w, tw, dangling, p, ar, s, alpha);
-        default: return launch_power<32>(n, in_off, in_src, in_w, tw, dangling, p, ar, s, alpha);
+        case 4: return launch_power<4>(n, m, in_off, in_src, in_w, tw, dangling, p, ar, s, alpha);
+        case 8: return launch_power<8>(n, m, in_off, in_src, in_w, tw, dangling, p, ar, s, alpha);
+        case 16: return launch_power<16>(n, m, in_off, in_src, in_w, tw, dangling, p, ar, s, alpha);
+        default: return launch_power<32>(n, m, in_off, in_src, in_w, tw, dangling, p, ar, s, alpha);
     }
 }
 

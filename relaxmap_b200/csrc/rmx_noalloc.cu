@@ -73,7 +73,7 @@ extern "C" rmx_status rmx_steady_state_noalloc(int32_t n_nodes, int64_t n_links,
         // without one, to the last word of the scratch. Every scratch word is
         // written by the solve before it is read, so nothing is cleared.
         int *iters = iters_out ? reinterpret_cast<int *>(iters_out) : reinterpret_cast<int *>(parts + 3 * kMaxBlocks);
-        rmx::power_iteration_into(n_nodes, in_off, in_src, in_w, teleport, dangling, p_out, y, parts, kMaxBlocks,
+        rmx::power_iteration_into(n_nodes, n_links, in_off, in_src, in_w, teleport, dangling, p_out, y, parts, kMaxBlocks,
                                   iters, static_cast<cudaStream_t>(stream),
                                   rmx::spmv_width((double)n_links / n_nodes));
     } catch (const std::exception &e) {

@@ -181,3 +181,38 @@ def test_flow_with_weighted_out_degree_hubs(built_lib, oracle_mod):
     assert rel(got["f"], st["f"]) <= 1e-12
     assert rel(got["exit"], st["exit"]) <= 1e-12
     assert abs(got["L0"] - st["L0"]) <= 1e-10
+
+
+def _flow_error(O, src, dst, w, n):
+    from relaxmap_b200 import Graph
+    st = O.initiate(O.prepare(O.from_edges(n, src, dst, w)))
+    with Graph.from_edges(src, dst, w, n=n) as G:
+        r = G.initiate()
+    return rel_l1(r["p"], st["p"])
+
+
+@pytest.mark.parametrize("n,deg", [(2, 1), (255, 3), (256, 9), (257, 20), (1000, 40), (4096, 20), (4097, 20),
+                                   (8192, 7), (8193, 7)])
+def test_small_graph_flow(built_lib, oracle_mod, n, deg):
+    """Sizes around the bounds of the one-cluster form of the power iteration (virtual blocks of
+    256 threads, 128 of them, 8192 nodes); dangling nodes among them."""
+    rng = np.random.default_rng(n)
+    src, dst = rng.integers(0, max(1, n - n // 10), n * deg), rng.integers(0, n, n * deg)
+    src[0], dst[0] = 0, n - 1
+    key = np.unique((src * np.int64(n) + dst)[src != dst])
+    src, dst = (key // n).astype(np.int32), (key % n).astype(np.int32)
+    assert _flow_error(oracle_mod, src, dst, rng.uniform(1, 10, len(src)), n) <= 1e-12
+
+
+@pytest.mark.parametrize("hub", [256, 257, 2999])
+def test_small_graph_flow_with_hub(built_lib, oracle_mod, hub):
+    """In-degrees on both sides of the bound (64 steps of 4 lanes) above which a small graph goes to
+    the grid form and its chunked rows."""
+    n = 3000
+    rng = np.random.default_rng(hub)
+    m = 6 * n
+    src = np.concatenate([np.arange(1, hub + 1), rng.integers(0, n, m)])
+    dst = np.concatenate([np.zeros(hub, dtype=np.int64), rng.integers(1, n, m)])
+    key = np.unique((src * np.int64(n) + dst)[src != dst])
+    src, dst = (key // n).astype(np.int32), (key % n).astype(np.int32)
+    assert _flow_error(oracle_mod, src, dst, None, n) <= 1e-12
