@@ -20,6 +20,15 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 const double kLn2 = std::log(2.0);
+// Largest source level converted in one launch. On the levels of the planted
+// graph of 20,011 nodes (209,114 links) it takes 0.12 ms against 0.26 ms by
+// separate kernels, on those of 150,001 nodes (2.5 to 2.9 million links) 0.45
+// against 0.44 ms, on those of 1M nodes (19 million) 1.6 against 1.2 ms: there
+// 16 warps per SM keep fewer links in flight than the separate kernels.
+#ifndef RMX_CONVERT_MAX
+#define RMX_CONVERT_MAX (1 << 20)
+#endif
+constexpr int64_t kConvertMaxLinks = RMX_CONVERT_MAX;
 
 __global__ void k_fill(double *a, int64_t n, double v) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -715,9 +724,13 @@ void rmx_graph::ensure_hub_table(const Level &lv) {
     level_hubs = 0;
     if (lv.n <= 0) return;
     int64_t need[4];
-    hub_level_needs(lv, need, dtmp + 12, stream);
+    if (&lv == known_lv && known_tuning == eval_tuning_generation())
+        std::copy(known_hub, known_hub + 4, need);  // counted when the level was built
+    else
+        hub_level_needs(lv, need, dtmp + 12, stream);
     const int64_t units = need[0], parts = need[1], links = need[2], chunks = need[3];
     level_hubs = units;
+    if (&lv == &node_lv) node_hubs = units;
     if (units == 0 || (units <= work.hub_units && parts <= work.hub_parts && links <= work.hub_links &&
                        chunks <= work.hub_chunks))
         return;
@@ -941,16 +954,14 @@ void rmx_graph::stage_sweeps(Level &lv, bool allow_new, std::vector<double> &L, 
     const bool prior = opt.prior != 0;
     const double vthresh = prior ? -opt.vthresh : 0.0;  // OmpRelaxmap.cpp:66, Module.cpp:1490 vs :1127
     int64_t n_active = lv.n;
-    all_units(lv.n, work, stream);
     if (lv.n > 0) ensure_hub_table(lv);
     if (fused_ok(lv)) {
         if (!any_set(act) || opt.max_iter <= 0) return;
         set_active(act);
-        run_fused(lv, mods, inst1, prior, allow_new, false, vthresh, sub_batches_for(lv.n));
-        RMX_CUDA(cudaMemcpyAsync(L.data(), inst1.L, sizeof(double) * K, cudaMemcpyDeviceToHost, stream));
-        RMX_CUDA(cudaStreamSynchronize(stream));
+        run_fused(lv, mods, inst1, prior, allow_new, false, vthresh, sub_batches_for(lv.n), L.data());
         return;
     }
+    all_units(lv.n, work, stream);
     if (stage_graph_ok(lv)) {
         stage_sweeps_graph(lv, allow_new, L, act);
         return;
@@ -978,16 +989,18 @@ void rmx_graph::stage_sweeps(Level &lv, bool allow_new, std::vector<double> &L, 
 // A stage runs as one cooperative launch on levels without hub units, never
 // with profiling events or per-sweep printing.
 bool rmx_graph::fused_ok(const Level &lv) const {
-    return level_hubs == 0 && !timers.on && opt.verbose < 2 && lv.n > 0;
+    return level_hubs == 0 && !timers.on && opt.verbose < 2 && lv.n > 0 &&
+           scratch.cap - scratch.mark() >= fused_stage_bytes(lv.n);
 }
 
 // One stage as one launch (fused_stage), its sweeps and stamps counted on.
 void rmx_graph::run_fused(Level &lv, ModState &M, InstState &I, bool prior, bool allow_new, bool subtune,
-                          double vthresh, int ns) {
+                          double vthresh, int ns, double *L) {
     const FusedStage f{prior ? 1 : 0, allow_new ? 1 : 0, subtune ? 1 : 0, opt.max_iter, ns,    vthresh,
                        opt.threshold, kLn2,              run_seed,         stamp,        sweep_no};
     fused_stage(lv, M, I, work, f, stage_ctl, scratch, stream);
     int64_t sweeps = 0;
+    if (L) RMX_CUDA(cudaMemcpyAsync(L, I.L, sizeof(double) * I.n, cudaMemcpyDeviceToHost, stream));
     RMX_CUDA(cudaMemcpyAsync(&sweeps, stage_ctl, sizeof sweeps, cudaMemcpyDeviceToHost, stream));
     RMX_CUDA(cudaStreamSynchronize(stream));
     sweep_no += (uint64_t)sweeps;
@@ -1154,6 +1167,16 @@ void rmx_graph::project_sn_to_nodes() {
 void rmx_graph::convert_to_supernodes(bool from_sn) {
     const NvtxRange range("rmx coarsen");
     timers.begin(kTimerCoarsen, stream);
+    const int64_t hubs = !from_sn ? node_hubs : &sn() == known_lv ? known_hub[0] : 1;
+    known_lv = nullptr;
+    {
+        Level &from = from_sn ? sn() : node_lv;
+        if (convert_level(from, hubs, from_sn ? from.mod : nullptr, sn_buf[1 - sn_cur], nmod, mods, false)) {
+            sn_cur = 1 - sn_cur;
+            timers.end(kTimerCoarsen, stream);
+            return;
+        }
+    }
     count_units(node_lv, mods, stream);  // nodes per module
     size_t mk = scratch.mark();
     int64_t *snid = scratch.alloc<int64_t>(N + 1);
@@ -1188,6 +1211,23 @@ void rmx_graph::convert_to_supernodes(bool from_sn) {
     sn_cur = 1 - sn_cur;
     count_units(sn(), mods, stream);
     timers.end(kTimerCoarsen, stream);
+}
+
+// The conversion as one launch, for source levels of up to kConvertMaxLinks
+// links and no hub units (the modules around hubs gather more links than its
+// tables take); false if it was not done.
+bool rmx_graph::convert_level(Level &from, int64_t from_hubs, const int32_t *row_mod, Level &to, const int32_t *unit_mod, ModState &M,
+                              bool sub) {
+    if (from.m > kConvertMaxLinks || from.m <= 0 || from_hubs > 0) return false;
+    const ConvertArgs c{N, K, sub, unit_mod, &M, mods.inst, &from, from.m, row_mod, &to, node_sn};
+    ConvertResult r;
+    if (!convert_fused(c, r, scratch, stream)) return false;
+    to.n = r.n;
+    to.m = r.m;
+    known_lv = &to;
+    known_tuning = eval_tuning_generation();
+    std::copy(r.hub, r.hub + 4, known_hub);
+    return true;
 }
 
 // generate_sub_modules (OmpRelaxmap.cpp:502-638): every module becomes an
@@ -1243,7 +1283,7 @@ void rmx_graph::generate_sub_modules() {
         timers.begin(kTimerLvSub, stream);
         const int nsg = sub_batches_for(N);
         const bool fused = fused_ok(sub_lv);
-        if (fused && opt.max_iter > 0) run_fused(sub_lv, submods, instsub, false, false, true, 0.0, nsg);
+        if (fused && opt.max_iter > 0) run_fused(sub_lv, submods, instsub, false, false, true, 0.0, nsg, nullptr);
         if (!fused && stage_graph_ok(sub_lv) && opt.max_iter > 0) {
             const StageGraphKey key{&sub_lv, &submods, &instsub, 0, 0, opt.max_iter, nsg, 0.0, opt.threshold,
                                     work.hub_gen, eval_tuning_generation(), scratch.mark()};
@@ -1272,6 +1312,11 @@ void rmx_graph::generate_sub_modules() {
     }
     // sub-modules -> super-nodes (generateSuperNodesFromSubModules, Module.cpp:3083-3158)
     timers.begin(kTimerCoarsen, stream);
+    known_lv = nullptr;
+    if (convert_level(node_lv, node_hubs, nullptr, sn(), submod, submods, true)) {
+        timers.end(kTimerCoarsen, stream);
+        return;
+    }
     count_units(sub_lv, submods, stream);
     mk = scratch.mark();
     int64_t *snid = scratch.alloc<int64_t>(N + 1);

@@ -221,6 +221,13 @@ void configure_eval_kernels();
 // (out[0..3]); one device reduction, then a sync.
 void hub_level_needs(const Level &L, int64_t *out, int64_t *dev_tmp, cudaStream_t s);
 
+// What hub_level_needs counts: units above bound, parts of part links (at most
+// max_parts), chunks of chunk links.
+struct HubNeeds {
+    int64_t bound, part, chunk, max_parts;
+};
+HubNeeds hub_needs_rule();
+
 // Launch shape of move evaluation, process-wide and read at every launch:
 // the grid cap of each bin in blocks per SM, and the degree bounds that
 // assign units to the warp, mid, block and large bins (units above large_max
@@ -270,6 +277,7 @@ struct FusedStage {
     uint32_t run_seed, stamp;     // stamp: of the last sub-batch so far
     uint64_t sweep_no;            // sweeps so far
 };
+size_t fused_stage_bytes(int32_t n);  // scratch it needs for a level of n units
 void fused_stage(const Level &lv, ModState &M, InstState &I, SweepWork &W, const FusedStage &f, int64_t *ctl, Arena &ar,
                  cudaStream_t s);
 // Move evaluation only, for the parity hook (no commit).
@@ -297,6 +305,31 @@ int64_t aggregate_links(int32_t n, const int64_t *off, const int32_t *dst, const
                         int32_t *g_out_src, int64_t *g_in_off, int32_t *g_in_src, fx_t *g_in_fx, fx_t *rowsum,
                         Arena &gtab_arena, fx_t *&gtab, int64_t &gtab_cap, Arena &ar, cudaStream_t s,
                         const SweepWork *W);
+// A partition's next super-node level as one cooperative launch
+// (rmx_convert.cu): super-nodes numbered by ascending module id with the
+// module's statistics, the source level's links between groups summed, node_sn,
+// and the units per module of the new level in M->count (its nodes in the sub
+// form). False: a group has too many links for the kernel's tables; nothing is
+// kept and the caller converts through aggregate_links.
+struct ConvertArgs {
+    int32_t N;
+    int K;
+    bool sub;                    // sub-modules of the coarse-tune: the super-node's module is its parent's
+    const int32_t *unit_mod;     // module of every node
+    const ModState *M;           // those modules
+    const int32_t *parent_inst;  // sub: instance of every parent module
+    const Level *src;            // links to sum, m of them
+    int64_t m;
+    const int32_t *row_mod;      // module of every unit of src, or null if its units are the nodes
+    Level *dst;
+    int32_t *node_sn;
+};
+struct ConvertResult {
+    int32_t n = 0;
+    int64_t m = 0;
+    int64_t hub[4] = {};  // as hub_level_needs
+};
+bool convert_fused(const ConvertArgs &c, ConvertResult &out, Arena &ar, cudaStream_t s);
 // src[e] = the row of link e for the CSR offsets off[0..n] (a warp per row).
 void rows_of_links(int32_t n, const int64_t *off, int32_t *src, cudaStream_t s);
 

@@ -111,6 +111,11 @@ struct rmx_graph {
     rmx::Arena hub_arena, agg_arena;
     rmx::fx_t *agg_tab = nullptr;
     int64_t agg_cap = 0;
+    // the level convert_level last built, and what its hub units need
+    const rmx::Level *known_lv = nullptr;
+    int64_t known_hub[4] = {};
+    int known_tuning = 0;
+    int64_t node_hubs = 0;   // hub units of the node level
     int64_t level_hubs = 0;  // hub units of the level ensure_hub_table last saw
 
     // ---- instances: 1 for a single graph; a batch is a disjoint union of
@@ -191,7 +196,7 @@ struct rmx_graph {
                       std::vector<double> &L);
     bool fused_ok(const rmx::Level &lv) const;
     void run_fused(rmx::Level &lv, rmx::ModState &M, rmx::InstState &I, bool prior, bool allow_new, bool subtune,
-                   double vthresh, int ns);
+                   double vthresh, int ns, double *L);
     bool stage_graph_ok(const rmx::Level &lv) const;
     void stage_sweeps_graph(rmx::Level &lv, bool allow_new, std::vector<double> &L, const std::vector<uint8_t> &act);
     void stage_body(rmx::Level &lv, bool allow_new, bool prior, double vthresh, int ns, unsigned long long cond);
@@ -202,6 +207,8 @@ struct rmx_graph {
                         const rmx::SweepArgs &sa, int ns, bool mark, uint32_t seed);
     int union_flows();
     void convert_to_supernodes(bool from_sn);
+    bool convert_level(rmx::Level &from, int64_t from_hubs, const int32_t *row_mod, rmx::Level &to, const int32_t *unit_mod,
+                       rmx::ModState &M, bool sub);
     void generate_sub_modules();
     void project_sn_to_nodes();
     int32_t count_modules();

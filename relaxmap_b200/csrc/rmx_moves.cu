@@ -1387,6 +1387,11 @@ __global__ void k_hub_level(int32_t n, const int64_t *out_off, const int64_t *in
     }
 }
 
+HubNeeds hub_needs_rule() {
+    const EvalTuning t = eval_tuning();
+    return {t.large_max, t.hub_part, kHubCh, kMaxParts};
+}
+
 void hub_level_needs(const Level &L, int64_t *out, int64_t *dev_tmp, cudaStream_t s) {
     unsigned long long *acc = reinterpret_cast<unsigned long long *>(dev_tmp);
     RMX_CUDA(cudaMemsetAsync(acc, 0, 4 * sizeof(unsigned long long), s));

@@ -998,6 +998,10 @@ __global__ void __launch_bounds__(kSwT, RMX_STAGE_MINB) k_stage(const __grid_con
 
 }  // namespace
 
+size_t fused_stage_bytes(int32_t n) {
+    return (size_t)n * (sizeof(URec) + sizeof(int32_t)) + 2 * sizeof(SweepSet) + (1 << 16);
+}
+
 void fused_stage(const Level &lv, ModState &M, InstState &I, SweepWork &W, const FusedStage &f, int64_t *ctl, Arena &ar,
                  cudaStream_t s) {
     static std::mutex mu;

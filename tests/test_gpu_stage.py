@@ -1,6 +1,10 @@
-"""The stage of sweeps as one launch against the same stage as separate
+"""Stages and conversions as one launch.
+
+The stage of sweeps as one launch against the same stage as separate
 kernels (per-sweep printing selects those): same decisions, exact integer
-sums, so partitions, code lengths and sweep counts are equal bit for bit."""
+sums, so partitions, code lengths and sweep counts are equal bit for bit.
+The conversion to super-nodes: link sums equal to the exact integer sums of
+the members' links, on groups around every bound between two team sizes."""
 import numpy as np
 import pytest
 
@@ -61,3 +65,40 @@ def test_one_launch_equals_kernels(built_lib, case, nsub, prior, capfd):
     assert one["L"] == kernels["L"]
     assert np.array_equal(one["steps_bits"], kernels["steps_bits"])
     assert np.array_equal(one["part"], kernels["part"])
+
+
+@pytest.mark.parametrize("links", [1, 255, 256, 257, 1023, 1024, 1025, 4095, 4096, 4097, 8193, 16383, 16384, 16385])
+def test_conversion_of_a_group_of(built_lib, links):
+    """One module with the given number of links to other modules, all of them distinct, among small ones."""
+    from relaxmap_b200 import Graph
+    members, others = 48, 17000
+    n = members + others
+    rng = np.random.default_rng(links)
+    to = members + rng.permutation(others)[:links]
+    src = np.concatenate([np.arange(links) % members, np.arange(members), members + np.arange(others)])
+    dst = np.concatenate([to, (np.arange(members) + 1) % members, members + (np.arange(others) * 7 + 3) % others])
+    keep = src != dst
+    src, dst = src[keep], dst[keep]
+    part = np.concatenate([np.zeros(members), members + np.arange(others) // 2 * 2]) if links % 2 else \
+        np.concatenate([np.zeros(members), members + np.arange(others)])
+    part = part.astype(np.int32)
+    with Graph.from_edges(src, dst, rng.uniform(1, 3, len(src)), n=n) as g:
+        off, gdst, _, _ = g.links()
+        f = g.initiate()["f"]
+        c = g.coarsen_engine(part)
+    fx = np.rint(f * 2.0 ** 62).astype(np.int64)
+    group = c["sn_of_mod"][part].astype(np.int64)
+    a, b = np.repeat(group, np.diff(off)), group[gdst]
+    cross = a != b
+    key, at = np.unique(a[cross] * c["n_sn"] + b[cross], return_inverse=True)
+    want = np.zeros(len(key), dtype=np.int64)
+    np.add.at(want, at, fx[cross])
+    assert c["n_sn"] == len(np.unique(part)) and len(c["out_dst"]) == len(key)
+    rows = np.repeat(np.arange(c["n_sn"], dtype=np.int64), np.diff(c["out_off"]))
+    got = rows * c["n_sn"] + c["out_dst"]
+    order = np.argsort(got)
+    assert np.array_equal(got[order], key) and np.array_equal(c["out_fx"][order], want)
+    cols = np.repeat(np.arange(c["n_sn"], dtype=np.int64), np.diff(c["in_off"]))
+    got = c["in_src"].astype(np.int64) * c["n_sn"] + cols
+    order = np.argsort(got)
+    assert np.array_equal(got[order], key) and np.array_equal(c["in_fx"][order], want)
