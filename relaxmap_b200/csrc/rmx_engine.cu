@@ -986,10 +986,19 @@ void rmx_graph::stage_sweeps(Level &lv, bool allow_new, std::vector<double> &L, 
     timers.end(lvt, stream);
 }
 
-// A stage runs as one cooperative launch on levels without hub units, never
-// with profiling events or per-sweep printing.
+// Largest level whose stages run as one launch: with more links a sub-batch's
+// evaluation lasts long enough that its 16 warps per SM lose more against the
+// separate kernels' 32 than their launches cost (planted graphs, whole runs: 4.75
+// million links 75 ms as one launch against 80 ms, 7.6 million 157 against 159,
+// 11.4 million 307 against 304, 19 million 293 against 275). A union of
+// instances keeps to one launch: its instances stop one by one, so most of its
+// sweeps are short (160 copies, 27 million links: 217 against 255 ms).
+constexpr int64_t kFusedMaxLinks = 1 << 23;
+
+// A stage runs as one cooperative launch on levels without hub units and of
+// moderate size, never with profiling events or per-sweep printing.
 bool rmx_graph::fused_ok(const Level &lv) const {
-    return level_hubs == 0 && !timers.on && opt.verbose < 2 && lv.n > 0 &&
+    return level_hubs == 0 && (K > 1 || lv.m <= kFusedMaxLinks) && !timers.on && opt.verbose < 2 && lv.n > 0 &&
            scratch.cap - scratch.mark() >= fused_stage_bytes(lv.n);
 }
 

@@ -61,56 +61,56 @@ struct EvalArgs {
     int mark;
 };
 
-// Decide and write the proposal for unit u given the argmin over candidates.
-__device__ __forceinline__ int32_t finish_unit(const EvalArgs &a, int32_t u, const UnitCtx &c, double best,
-                                               int32_t bm) {
-    bool allow = a.allow_new_unit ? a.allow_new_unit[u] != 0 : (a.allow_new && a.mcount[c.A] > 1);
+// Decides unit u's proposal from the argmin over its candidates; writer: the
+// lane that stores it. new_exit, new_stay: plogp of the empty-module option's
+// exit and stay terms. Whether the unit found a move below the threshold: it
+// then activates its neighbours for the next prioritised sweep, whether or not
+// the move is taken (Module.cpp:1661-1668).
+__device__ __forceinline__ bool finish_unit(const EvalArgs &a, int32_t u, const UnitCtx &c, double new_exit,
+                                            double new_stay, double best, int32_t bm, bool writer) {
+    const int32_t nA = a.mcount[c.A];
+    const bool allow = a.allow_new_unit ? a.allow_new_unit[u] != 0 : (a.allow_new && nA > 1);
     if (allow) {
-        double dn = newmod_delta(c);
+        const double dn = plogp_total(c, c.eu) + c.K - 2.0 * new_exit + new_stay;
         if (better(dn, INT_MAX, best, bm)) {
             best = dn;
             bm = kNewMod;
         }
     }
-    int32_t out = -1;
-    if (bm != INT_MAX && best < a.vthresh) {
-        out = bm;
+    const bool act = bm != INT_MAX && best < a.vthresh;
+    if (writer) {
+        int32_t out = act ? bm : -1;
         // A singleton never moves into another singleton with a larger id: the
         // pair then merges in one direction instead of swapping.
-        if (a.swap_guard && bm >= 0 && a.mcount[c.A] == 1 && a.mcount[bm] == 1 && bm > c.A) out = -1;
+        if (act && a.swap_guard && bm >= 0 && nA == 1 && a.mcount[bm] == 1 && bm > c.A) out = -1;
+        a.prop[u] = out;
+        a.pdelta[u] = best;
     }
-    a.prop[u] = out;
-    a.pdelta[u] = best;
-    // a unit that found a move below the threshold activates its neighbours
-    // for the next prioritised sweep, whether or not the move is then taken
-    // (Module.cpp:1661-1668)
-    return (bm != INT_MAX && best < a.vthresh) ? 1 : 0;
-}
-
-// Mark every out/in neighbour of u active (a group of NT threads, rank r).
-template <int NT>
-__device__ __forceinline__ void mark_neighbours(const EvalArgs &a, int32_t u, int r) {
-    const int64_t ob = a.out_off[u], oe = a.out_off[u + 1], ib = a.in_off[u], ie = a.in_off[u + 1];
-    for (int64_t e = ob + r; e < oe; e += NT) a.next_active[a.out_dst[e]] = 1;
-    for (int64_t e = ib + r; e < ie; e += NT) a.next_active[a.in_src[e]] = 1;
+    return act;
 }
 
 // ---------------------------------------------------------------- evaluation
 // Degree bins (out+in degree d of the unit at this level):
-//   reg    d <= 32    8, 16 or 32 lanes per unit, one link per lane: the
-//                     group sorts (module, flows) by module with a bitonic
-//                     network and sums equal runs with a segmented scan, all
-//                     in registers; each run's last lane is one candidate
-//   warp   d <= 128   one warp per unit, table of <= 256 slots per warp in
-//                     shared memory, candidates compacted in place
-//   block  d <= 1024  256 threads per unit, table of <= 2048 slots in shared memory
-//   large  d <= 4096  512 threads per unit, table of <= 8192 slots in shared memory
-//   hub    d > 4096   512 threads per unit, table in a per-block slice of a
-//                     global table (one block per SM)
-// Each unit: clear the table, insert every link's neighbour module with its
-// fixed-point flow (integer atomics, so the sums do not depend on the order),
-// look up the own module, compact the other occupied slots in place into a
-// dense candidate list, and evaluate the candidates with all lanes.
+//   reg    d <= 32    8, 16 or 32 lanes per unit, one link per lane, 4 slots
+//                     per lane in shared memory
+//   warp   d <= 128   one warp per unit, 256 slots
+//   mid    d <= 512   128 threads per unit, 1024 slots
+//   block  d <= 1024  256 threads per unit, 2048 slots
+//   large  d <= 4096  512 threads per unit, 8192 slots
+//   hub    d > 4096   every unit split over many blocks (below)
+// Each unit's links are inserted with their fixed-point flow into a table keyed
+// by the neighbour's module (integer sums: exact in any order); whoever fills a
+// slot evaluates its module. Links to the unit's own module are summed in
+// registers. Bound by instruction issue and the latency of the random module
+// records: of 50 to 69 million warp instructions per sub-batch and bin on R-MAT
+// scale 20 (issue slots 51% busy in the register and mid bins) most are the two
+// FP64 logarithms per candidate. Sums as two 32-bit atomics, the unit's six
+// logarithms taken by six lanes in one call, slots listed as they are filled
+// instead of scanned for, and the next unit's offsets loaded ahead: evaluation
+// of a whole run 191 -> 155 ms on the 1M-node planted graph, 135 -> 121 ms on
+// R-MAT scale 22. Fetching each record into L2 from the insertion on was
+// slower (158 and 124 ms), and so was __match_any_sync instead of a table in
+// the register bin (58 cycles per warp and SM).
 
 constexpr int kWarpMaxDeg = 128, kWarpCap = 256, kEvalWarps = 8;
 // units of 129..512 links: four warps each (eight teams per SM), a 1024-slot table
@@ -152,19 +152,6 @@ constexpr int kBlkT = 256, kBlkMaxDeg = 1024, kBlkCap = 2048;
 #endif
 constexpr int kLrgT = 512, kLrgCap = RMX_LRG_CAP, kLrgMaxDeg = kLrgCap / 2;
 
-// Slot of key, or -1 (linear probing); keys[s * KS] is slot s's key.
-template <int KS = 1>
-__device__ __forceinline__ int tab_find(const int32_t *keys, int mask, int32_t key) {
-    int s = tab_slot(key, mask);
-    for (int probe = 0; probe <= mask; probe++) {
-        const int32_t k = keys[(int64_t)s * KS];
-        if (k == key) return s;
-        if (k == kEmpty) return -1;
-        s = (s + 1) & mask;
-    }
-    return -1;
-}
-
 template <int NT>
 __device__ __forceinline__ void gsync() {
     if (NT == 32)
@@ -177,127 +164,244 @@ template <int NT>
 struct GroupShared {  // reductions across the warps of a block group
     double best[NT / 32];
     int32_t mod[NT / 32];
-    int ncand;
+    fx_t sA[NT / 32];
 };
 
-// Inserts the unit's links j = first, first + NT, ... below end (out-links
-// first, then in-links; dout of them out) into the table keys/vals keyed by
-// the neighbour's module, adding each link's fixed-point flow to the slot's
-// sum. RMX_EVAL_ILP links at a time have their neighbour ids, flows and then
-// neighbour modules loaded before any is inserted, so that many gathers are in
-// flight per thread. Capacity >= 2 x the unit's links, so probing always
-// finds a slot.
-template <int NT>
-__device__ __forceinline__ void insert_links(const EvalArgs &a, int64_t ob, int64_t ib, int64_t dout, int64_t first,
-                                             int64_t d, int32_t *keys, fx_t *vals, int mask) {
-    for (int64_t j0 = first; j0 < d; j0 += (int64_t)RMX_EVAL_ILP * NT) {
+// A group's table: keys, the slots' fixed-point sums in two halves (32-bit
+// shared atomics are native, a 64-bit one is a loop of compare-and-swaps, a
+// sixth of the throughput), and the calling warp's list of slots it filled.
+struct Table {
+    int32_t *keys;
+    unsigned *lo, *hi;
+    uint16_t *list;
+};
+// Bytes of a table of cap slots with its lists (half as many entries as slots).
+__host__ __device__ constexpr size_t table_bytes(int cap) { return (size_t)cap * (3 * sizeof(int32_t)) + (size_t)cap / 2 * sizeof(uint16_t); }
+__device__ __forceinline__ Table table_at(unsigned char *p, int cap, int warps, int w) {
+    Table t;
+    t.keys = reinterpret_cast<int32_t *>(p);
+    t.lo = reinterpret_cast<unsigned *>(t.keys + cap);
+    t.hi = t.lo + cap;
+    t.list = reinterpret_cast<uint16_t *>(t.hi + cap) + w * (cap / 2 / warps);
+    return t;
+}
+__device__ __forceinline__ void table_clear(const Table &t, int cap, int r, int n) {
+    for (int s = r; s < cap; s += n) {
+        t.keys[s] = kEmpty;
+        t.lo[s] = t.hi[s] = 0;
+    }
+}
+__device__ __forceinline__ void table_add(const Table &t, int s, fx_t q) {
+    const unsigned ql = (unsigned)q, old = atomicAdd(t.lo + s, ql);
+    atomicAdd(t.hi + s, (unsigned)((unsigned long long)q >> 32) + (old + ql < old ? 1u : 0u));
+}
+// Slot s's sum; the slot is emptied.
+__device__ __forceinline__ fx_t table_take(const Table &t, int s) {
+    const fx_t v = (fx_t)(((unsigned long long)t.hi[s] << 32) | t.lo[s]);
+    t.keys[s] = kEmpty;
+    t.lo[s] = t.hi[s] = 0;
+    return v;
+}
+
+// What a unit's evaluation starts from, loaded while the unit before it is evaluated.
+struct UnitHead {
+    int32_t u, A;
+    uint32_t ob, ib;  // link offsets fit 32 bits: a graph has fewer than 2^31 links
+    int32_t dout, din;
+};
+__device__ __forceinline__ UnitHead load_head(const EvalArgs &a, int64_t i, int64_t end) {
+    UnitHead h;
+    h.u = -1;
+    if (i < end) {
+        h.u = a.list[i];
+        const int64_t ob = a.out_off[h.u], ib = a.in_off[h.u];
+        h.dout = (int32_t)(a.out_off[h.u + 1] - ob);
+        h.din = (int32_t)(a.in_off[h.u + 1] - ib);
+        h.ob = (uint32_t)ob;
+        h.ib = (uint32_t)ib;
+        h.A = a.mod[h.u];
+    }
+    return h;
+}
+
+// One unit evaluated by a group of NT threads (a warp or a block); r = rank.
+// Links j = r, r + NT, ... (out-links first): RMX_EVAL_ILP of them have their
+// neighbour ids, flows and then neighbour modules loaded before any is
+// inserted. Links to the unit's own module are summed in registers; for the
+// others the thread that fills a slot notes it in its warp's list. The table (CAP
+// slots, at least twice the unit's links) is empty before and after: each warp
+// empties the slots it filled while it evaluates them.
+template <int NT, int CAP>
+__device__ __forceinline__ void eval_unit(const EvalArgs &a, const UnitHead &h, const int r, const Table &t,
+                                          GroupShared<NT> *sh, unsigned long long &seen, unsigned long long &cands) {
+    constexpr int mask = CAP - 1;
+    const int lane = r & 31;
+    const int d = h.dout + h.din;
+    const uint32_t ibm = h.ib - (uint32_t)h.dout;
+    fx_t sA = 0;
+    int cnt = 0;
+    for (int j0 = 0; j0 < d; j0 += RMX_EVAL_ILP * NT) {
         int32_t key[RMX_EVAL_ILP];
         fx_t q[RMX_EVAL_ILP];
 #pragma unroll
         for (int k = 0; k < RMX_EVAL_ILP; k++) {
-            const int64_t j = j0 + (int64_t)k * NT;
             key[k] = -1;
             q[k] = 0;
-            if (j < d) {
-                const bool isout = j < dout;
-                const int64_t e = isout ? ob + j : ib + (j - dout);
+            if (j0 + k * NT < d) {  // the same in the whole group; lanes past the links read the last one
+                const int j = min(j0 + k * NT + r, d - 1);
+                const bool isout = j < h.dout;
+                const uint32_t e = (isout ? h.ob : ibm) + (uint32_t)j;
                 // links are streamed (evict-first) so that the module ids they point to stay in L2
-                key[k] = __ldcs(isout ? a.out_dst + e : a.in_src + e);
-                q[k] = __ldcs(isout ? a.out_fx + e : a.in_fx + e);
+                key[k] = __ldcs((isout ? a.out_dst : a.in_src) + e);
+                q[k] = __ldcs((isout ? a.out_fx : a.in_fx) + e);
             }
         }
 #pragma unroll
         for (int k = 0; k < RMX_EVAL_ILP; k++)
-            if (key[k] >= 0) key[k] = __ldg(a.mod + key[k]);
-        // first probes of all keys issued together, then each key's collisions
+            if (j0 + k * NT < d) key[k] = __ldg(a.mod + key[k]);
         int slot[RMX_EVAL_ILP];
         int32_t prev[RMX_EVAL_ILP];
 #pragma unroll
-        for (int k = 0; k < RMX_EVAL_ILP; k++)
-            if (key[k] >= 0) {
-                slot[k] = tab_slot(key[k], mask);
-                prev[k] = atomicCAS(keys + slot[k], kEmpty, key[k]);
+        for (int k = 0; k < RMX_EVAL_ILP; k++) {
+            if (j0 + k * NT + r >= d) key[k] = -1;
+            if (key[k] == h.A) {
+                sA += q[k];
+                key[k] = -1;
             }
+            slot[k] = tab_slot(key[k], mask);
+            prev[k] = 0;
+            if (key[k] >= 0) prev[k] = atomicCAS(t.keys + slot[k], kEmpty, key[k]);
+        }
+        // at least twice as many slots as links: a free one exists
+        for (int probe = 0; probe < mask; probe++) {
+            bool more = false;
 #pragma unroll
-        for (int k = 0; k < RMX_EVAL_ILP; k++)
-            if (key[k] >= 0) {
-                // capacity >= 2 x the unit's links: a free slot exists, probing stays below mask steps
-                for (int probe = 0; prev[k] != kEmpty && prev[k] != key[k] && probe < mask; probe++) {
+            for (int k = 0; k < RMX_EVAL_ILP; k++)
+                if (key[k] >= 0 && prev[k] != kEmpty && prev[k] != key[k]) {
                     slot[k] = (slot[k] + 1) & mask;
-                    prev[k] = atomicCAS(keys + slot[k], kEmpty, key[k]);
+                    prev[k] = atomicCAS(t.keys + slot[k], kEmpty, key[k]);
+                    more = true;
                 }
-                atomic_add_fx(vals + slot[k], q[k]);
-            }
-    }
-}
-
-// One unit evaluated by a group of NT threads (a warp or a block); r = rank.
-// The candidate list overwrites the table in place.
-template <int NT>
-__device__ __forceinline__ void eval_unit(const EvalArgs &a, const int32_t u, const int r, int32_t *keys, fx_t *vals,
-                                          GroupShared<NT> *sh, unsigned long long &seen, unsigned long long &cands) {
-    const int lane = r & 31;
-    const unsigned lt = (1u << lane) - 1u;
-    const int64_t ob = a.out_off[u], ib = a.in_off[u];
-    const int64_t dout = a.out_off[u + 1] - ob, d = dout + (a.in_off[u + 1] - ib);
-    int64_t cap = 32;
-    while (cap < 2 * d) cap <<= 1;
-    const int mask = (int)(cap - 1);
-    // The table is empty on entry: cleared once when the kernel starts (shared
-    // tables) or when it is allocated (global slices), and every unit leaves
-    // it empty again (below), so no clearing pass runs per unit.
-    insert_links<NT>(a, ob, ib, dout, r, d, keys, vals, mask);
-    gsync<NT>();
-    const int32_t A = a.mod[u];
-    const int sA = tab_find(keys, mask, A);
-    const UnitCtx c = make_ctx(a.attr[u], a.mrec[A], a.inst_sum_exit[a.uinst[u]], A,
-                               sA >= 0 ? vals[sA] : 0);
-    if (NT > 32) __syncthreads();  // every lookup is done before slots are overwritten
-    // Each warp compacts its own contiguous slice of the table in place (the
-    // dense position never passes the slot being read) and evaluates it. A
-    // slot left beyond the dense prefix is emptied at once; the prefix is
-    // emptied as its candidates are evaluated.
-    const int64_t seg = cap / (NT / 32), lo = (int64_t)(r >> 5) * seg, hi = lo + seg;
-    int nc = 0;
-    for (int64_t base = lo; base < hi; base += 32) {
-        const int64_t s = base + lane;
-        int32_t k = kEmpty;
-        fx_t v = 0;
-        if (s < hi) {
-            k = keys[s];
-            v = vals[s];
+            if (!more) break;
         }
-        const bool occ = k != kEmpty && k != A;
-        const unsigned bal = __ballot_sync(kFull, occ);
+#pragma unroll
+        for (int k = 0; k < RMX_EVAL_ILP; k++) {
+            const bool fresh = key[k] >= 0 && prev[k] == kEmpty;
+            if (key[k] >= 0) table_add(t, slot[k], q[k]);
+            const unsigned bal = __ballot_sync(kFull, fresh);
+            if (fresh) t.list[cnt + __popc(bal & ((1u << lane) - 1u))] = (uint16_t)slot[k];
+            cnt += __popc(bal);
+        }
+    }
+    const Stat4 ua = load_stat(a.attr + h.u);
+    const ModRec mA = load_mod(a.mrec + h.A);
+    const double DA = a.mrec[h.A].D;
+    const double se = a.inst_sum_exit[a.uinst[h.u]];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sA += __shfl_xor_sync(kFull, sA, o);
+    if (NT > 32) {
+        if (lane == 0) sh->sA[r >> 5] = sA;
+        __syncthreads();
+        sA = 0;
+#pragma unroll
+        for (int q = 0; q < NT / 32; q++) sA += sh->sA[q];
+    } else {
         __syncwarp();
-        if (occ) {
-            const int64_t p = lo + nc + __popc(bal & lt);
-            keys[p] = k;
-            vals[p] = v;
-        }
-        nc += __popc(bal);
-        if (k != kEmpty && s >= lo + nc) {  // not overwritten by the dense prefix
-            keys[s] = kEmpty;
-            vals[s] = 0;
-        }
     }
-    __syncwarp();
+    double new_exit, new_stay;
+    const UnitCtx c = make_ctx_lanes(32, ua, mA, DA, se, h.A, sA, lane, new_exit, new_stay);
     double best = 0.0;
     int32_t bm = INT_MAX;
-    for (int q = lane; q < nc; q += 32) {
-        const int32_t m = keys[lo + q];
-        const fx_t v = vals[lo + q];
-        keys[lo + q] = kEmpty;
-        vals[lo + q] = 0;
-        const double dl = candidate_delta(c, a.mrec[m], v);
+    for (int q = lane; q < cnt; q += 32) {
+        const int s = t.list[q];
+        const int32_t m = t.keys[s];
+        const ModRec rm = load_mod(a.mrec + m);
+        const double dl = candidate_delta(c, rm, table_take(t, s));
         if (better(dl, m, best, bm)) {
             best = dl;
             bm = m;
         }
     }
     // lanes without a candidate hold (0, INT_MAX), which no real candidate loses to
+    warp_best(best, bm);
+    if (NT > 32) {
+        if (lane == 0) {
+            sh->best[r >> 5] = best;
+            sh->mod[r >> 5] = bm;
+        }
+        __syncthreads();
+        best = lane < NT / 32 ? sh->best[lane] : 0.0;
+        bm = lane < NT / 32 ? sh->mod[lane] : INT_MAX;
+        warp_best(best, bm);
+    }
+    if (lane == 0) cands += cnt;
+    if (r == 0) seen += d;
+    const bool act = finish_unit(a, h.u, c, new_exit, new_stay, best, bm, r == 0);
+    if (a.mark && act)
+        for (int j = r; j < d; j += NT)
+            a.next_active[j < h.dout ? a.out_dst[h.ob + (uint32_t)j] : a.in_src[ibm + (uint32_t)j]] = 1;
+    if (NT == 32) __syncwarp();
+}
+
+// Group of W lanes per unit (d <= W), one link per lane: equal modules meet in
+// the group's slots (4 W from slot tb on) of the warp's table, and the lane that
+// filled a slot evaluates its module.
+template <int W>
+__device__ __forceinline__ void eval_unit_reg(const EvalArgs &a, const int32_t u, const bool valid, const int gl,
+                                              const Table &t, unsigned long long &seen, unsigned long long &cands) {
+    const int lane = threadIdx.x & 31, tb = (lane / W) * 4 * W;
+    constexpr int mask = 4 * W - 1;
+    int32_t nbr = 0, key = -1, A = 0;
+    fx_t v = 0;
+    int d = 0;
+    if (valid) {
+        const int64_t ob = a.out_off[u], ib = a.in_off[u];
+        const int dout = (int)(a.out_off[u + 1] - ob);
+        d = dout + (int)(a.in_off[u + 1] - ib);
+        A = a.mod[u];
+        if (gl < d) {
+            const bool isout = gl < dout;
+            const int64_t e = isout ? ob + gl : ib + (gl - dout);
+            nbr = __ldcs((isout ? a.out_dst : a.in_src) + e);  // links streamed, module ids kept
+            v = __ldcs((isout ? a.out_fx : a.in_fx) + e);
+            key = __ldg(a.mod + nbr);
+        }
+    }
+    const bool has = gl < d, other = has && key != A;
+    int slot = tb;
+    bool fresh = false;
+    ModRec rm;
+    if (other) {
+        rm = load_mod(a.mrec + key);
+        int s = tab_slot(key, mask);
+        int32_t prev = atomicCAS(t.keys + tb + s, kEmpty, key);
+        for (int probe = 0; prev != kEmpty && prev != key && probe < mask; probe++) {  // at most a quarter full
+            s = (s + 1) & mask;
+            prev = atomicCAS(t.keys + tb + s, kEmpty, key);
+        }
+        slot = tb + s;
+        fresh = prev == kEmpty;
+        table_add(t, slot, v);
+    }
+    const Stat4 ua = load_stat(a.attr + u);
+    const ModRec mA = load_mod(a.mrec + A);
+    const double DA = a.mrec[A].D;
+    const double se = a.inst_sum_exit[a.uinst[u]];
+    fx_t sA = has && !other ? v : 0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
+    for (int o = W / 2; o > 0; o >>= 1) sA += __shfl_xor_sync(kFull, sA, o);
+    __syncwarp();
+    double new_exit, new_stay;
+    const UnitCtx c = make_ctx_lanes(W, ua, mA, DA, se, A, sA, gl, new_exit, new_stay);
+    double best = 0.0;
+    int32_t bm = INT_MAX;
+    if (fresh) {
+        best = candidate_delta(c, rm, table_take(t, slot));
+        bm = key;
+    }
+    cands += fresh ? 1 : 0;
+#pragma unroll
+    for (int o = W / 2; o > 0; o >>= 1) {
         const double ob2 = __shfl_xor_sync(kFull, best, o);
         const int32_t om = __shfl_xor_sync(kFull, bm, o);
         if (better(ob2, om, best, bm)) {
@@ -305,131 +409,31 @@ __device__ __forceinline__ void eval_unit(const EvalArgs &a, const int32_t u, co
             bm = om;
         }
     }
-    if (NT > 32) {
-        if (lane == 0) {
-            sh->best[r >> 5] = best;
-            sh->mod[r >> 5] = bm;
-        }
-        __syncthreads();
-        if (r == 0)
-            for (int q = 1; q < NT / 32; q++)
-                if (better(sh->best[q], sh->mod[q], best, bm)) {
-                    best = sh->best[q];
-                    bm = sh->mod[q];
-                }
-    }
-    int act = 0;
-    if (lane == 0) cands += nc;
-    if (r == 0) {
-        act = finish_unit(a, u, c, best, bm);
-        seen += d;
-    }
-    if (a.mark) {
-        if (NT == 32) {
-            act = __shfl_sync(kFull, act, 0);
-        } else {
-            if (r == 0) sh->ncand = act;
-            __syncthreads();
-            act = sh->ncand;
-        }
-        if (act) mark_neighbours<NT>(a, u, r);
-    }
-    gsync<NT>();
-}
-
-// Group of W lanes per unit (d <= W), everything in registers.
-template <int W>
-__device__ __forceinline__ void eval_unit_reg(const EvalArgs &a, const int32_t u, const bool valid, const int gl,
-                                              const unsigned gmask, unsigned long long &seen,
-                                              unsigned long long &cands) {
-    int32_t key = INT_MAX, nbr = -1;
-    fx_t v = 0;
-    int64_t d = 0;
-    int32_t A = -1;
     if (valid) {
-        const int64_t ob = a.out_off[u], ib = a.in_off[u];
-        const int64_t dout = a.out_off[u + 1] - ob;
-        d = dout + (a.in_off[u + 1] - ib);
-        A = a.mod[u];
-        if (gl < d) {
-            const bool isout = gl < dout;
-            const int64_t e = isout ? ob + gl : ib + (gl - dout);
-            nbr = __ldcs(isout ? a.out_dst + e : a.in_src + e);  // links streamed, module ids kept
-            key = __ldg(a.mod + nbr);
-            v = __ldcs(isout ? a.out_fx + e : a.in_fx + e);
-        }
+        if (gl == 0) seen += d;
+        if (finish_unit(a, u, c, new_exit, new_stay, best, bm, gl == 0) && a.mark && has) a.next_active[nbr] = 1;
     }
-    // bitonic sort of (key, flow) by key within the group
-#pragma unroll
-    for (int k = 2; k <= W; k <<= 1) {
-#pragma unroll
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            const int32_t pk = __shfl_xor_sync(kFull, key, j, W);
-            const fx_t pv = __shfl_xor_sync(kFull, v, j, W);
-            const bool up = (gl & k) == 0, lower = (gl & j) == 0;
-            const bool take = lower == up ? pk < key : pk > key;
-            if (take) {
-                key = pk;
-                v = pv;
-            }
-        }
-    }
-    // sums over runs of equal keys (segmented inclusive scan)
-#pragma unroll
-    for (int off = 1; off < W; off <<= 1) {
-        const int32_t k2 = __shfl_up_sync(kFull, key, off, W);
-        const fx_t v2 = __shfl_up_sync(kFull, v, off, W);
-        if (gl >= off && k2 == key) v += v2;
-    }
-    const int32_t nk = __shfl_down_sync(kFull, key, 1, W);
-    const bool tail = key != INT_MAX && (gl == W - 1 || nk != key);
-    // the flow to and from the unit's own module from the lane ending A's run
-    const unsigned own = __ballot_sync(kFull, tail && key == A) & gmask;
-    const int src = own ? __ffs(own) - 1 : (threadIdx.x & 31);
-    fx_t sA = __shfl_sync(kFull, v, src);
-    if (!own) sA = 0;
-    double best = 0.0;
-    int32_t bm = INT_MAX;
-    UnitCtx c;
-    if (valid) {
-        c = make_ctx(a.attr[u], a.mrec[A], a.inst_sum_exit[a.uinst[u]], A, sA);
-        if (tail && key != A) {
-            best = candidate_delta(c, a.mrec[key], v);
-            bm = key;
-        }
-    }
-    const unsigned ncand = __popc(__ballot_sync(kFull, tail && key != A) & gmask);
-#pragma unroll
-    for (int o = W / 2; o > 0; o >>= 1) {
-        const double ob2 = __shfl_xor_sync(kFull, best, o, W);
-        const int32_t om = __shfl_xor_sync(kFull, bm, o, W);
-        if (better(ob2, om, best, bm)) {
-            best = ob2;
-            bm = om;
-        }
-    }
-    int act = 0;
-    if (valid && gl == 0) {
-        act = finish_unit(a, u, c, best, bm);
-        seen += d;
-        cands += ncand;
-    }
-    if (a.mark) {
-        act = __shfl_sync(kFull, act, (threadIdx.x & 31) & ~(W - 1));
-        if (act && nbr >= 0) a.next_active[nbr] = 1;
-    }
+    __syncwarp();
 }
 
 // Bins reg8, reg16, reg32: ranges range[0..3) of consecutive buckets.
 __global__ void __launch_bounds__(256, RMX_REG_MINB) k_eval_reg(EvalArgs a) {
+    constexpr int kRegCap = 128;  // slots per warp: four per lane
+    __shared__ __align__(16) unsigned char regtab[8][kRegCap * 12];
     const int lane = threadIdx.x & 31;
+    Table t;
+    t.keys = reinterpret_cast<int32_t *>(regtab[threadIdx.x >> 5]);
+    t.lo = reinterpret_cast<unsigned *>(t.keys + kRegCap);
+    t.hi = t.lo + kRegCap;
+    t.list = nullptr;
+    table_clear(t, kRegCap, lane, 32);
+    __syncwarp();
     const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
     unsigned long long seen = 0, units = 0, cands = 0;
 #define RMX_REG_BIN(W, b)                                                                       \
     {                                                                                           \
         const int64_t beg = a.range[b], end = a.range[b + 1];                                   \
         const int g = lane / W, gl = lane % W;                                                  \
-        const unsigned gmask = (W == 32 ? kFull : ((1u << W) - 1u)) << (g * W);                 \
         for (int64_t base = beg + gw * (32 / W); base < end; base += nw * (32 / W)) {           \
             const int64_t i = base + g;                                                         \
             bool valid = i < end;                                                               \
@@ -438,7 +442,7 @@ __global__ void __launch_bounds__(256, RMX_REG_MINB) k_eval_reg(EvalArgs a) {
                 if (gl == 0) a.prop[u] = -1;                                                    \
                 valid = false;                                                                  \
             }                                                                                   \
-            eval_unit_reg<W>(a, u, valid, gl, gmask, seen, cands);                              \
+            eval_unit_reg<W>(a, u, valid, gl, t, seen, cands);                                  \
             if (valid && gl == 0) units++;                                                      \
         }                                                                                       \
     }
@@ -476,25 +480,24 @@ __device__ __forceinline__ void flush_stats_split(const EvalArgs &a, unsigned lo
 }
 
 __global__ void __launch_bounds__(kEvalWarps * 32, RMX_WARP_MINB) k_eval_warp(EvalArgs a) {
-    __shared__ int32_t skey[kEvalWarps][kWarpCap];
-    __shared__ fx_t sval[kEvalWarps][kWarpCap];
+    __shared__ __align__(16) unsigned char tabs[kEvalWarps][table_bytes(kWarpCap)];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t beg = a.range[0], end = a.range[1];
     const int64_t gw = (int64_t)blockIdx.x * kEvalWarps + w, nw = (int64_t)gridDim.x * kEvalWarps;
     unsigned long long seen = 0, units = 0, cands = 0;
-    for (int s = lane; s < kWarpCap; s += 32) {  // every unit leaves its table empty again
-        skey[w][s] = kEmpty;
-        sval[w][s] = 0;
-    }
+    const Table t = table_at(tabs[w], kWarpCap, 1, 0);
+    table_clear(t, kWarpCap, lane, 32);
     __syncwarp();
+    UnitHead h = load_head(a, beg + gw, end);
     for (int64_t i = beg + gw; i < end; i += nw) {
-        const int32_t u = a.list[i];
-        if (!a.inst_active[a.uinst[u]]) {
-            if (lane == 0) a.prop[u] = -1;
-            continue;
+        const UnitHead next = load_head(a, i + nw, end);
+        if (a.inst_active[a.uinst[h.u]]) {
+            eval_unit<32, kWarpCap>(a, h, lane, t, nullptr, seen, cands);
+            units++;
+        } else if (lane == 0) {
+            a.prop[h.u] = -1;
         }
-        eval_unit<32>(a, u, lane, skey[w], sval[w], nullptr, seen, cands);
-        units++;
+        h = next;
     }
     if (lane == 0) flush_stats(a, seen, units, cands);
 }
@@ -506,23 +509,21 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? RMX_LRG_MINB : (NT == 128 ? 8 
     k_eval_block(EvalArgs a) {
     extern __shared__ __align__(16) unsigned char dsm[];
     __shared__ GroupShared<NT> sh;
-    fx_t *vals = reinterpret_cast<fx_t *>(dsm);
-    int32_t *keys = reinterpret_cast<int32_t *>(vals + CAP);
-    for (int s = threadIdx.x; s < CAP; s += NT) {  // every unit leaves its table empty again
-        keys[s] = kEmpty;
-        vals[s] = 0;
-    }
+    const Table t = table_at(dsm, CAP, NT / 32, threadIdx.x >> 5);
+    table_clear(t, CAP, threadIdx.x, NT);
     __syncthreads();
     const int64_t beg = a.range[0], end = a.range[1];
     unsigned long long seen = 0, units = 0, cands = 0;
+    UnitHead h = load_head(a, beg + blockIdx.x, end);
     for (int64_t i = beg + blockIdx.x; i < end; i += gridDim.x) {
-        const int32_t u = a.list[i];
-        if (!a.inst_active[a.uinst[u]]) {
-            if (threadIdx.x == 0) a.prop[u] = -1;
-            continue;
+        const UnitHead next = load_head(a, i + gridDim.x, end);
+        if (a.inst_active[a.uinst[h.u]]) {
+            eval_unit<NT, CAP>(a, h, threadIdx.x, t, &sh, seen, cands);
+            units++;
+        } else if (threadIdx.x == 0) {
+            a.prop[h.u] = -1;
         }
-        eval_unit<NT>(a, u, threadIdx.x, keys, vals, &sh, seen, cands);
-        units++;
+        h = next;
     }
     // every warp found its own share of the candidates; thread 0 alone counted the links
     if ((threadIdx.x & 31) == 0) flush_stats_split(a, threadIdx.x == 0 ? seen : 0, threadIdx.x == 0 ? units : 0, cands);
@@ -811,8 +812,12 @@ __global__ void __launch_bounds__(1024) k_hub_offsets(HubPlan p) {
 // overfills (at R = 2^31 a round holds at most two keys).
 __global__ void __launch_bounds__(kHubPT, RMX_HUB_MINB) k_hub_eval(EvalArgs a, HubPlan p) {
     extern __shared__ __align__(16) unsigned char hub_smem[];  // kHubEvalSmem bytes
-    fx_t *vals = reinterpret_cast<fx_t *>(hub_smem);
-    int32_t *keys = reinterpret_cast<int32_t *>(vals + kPartCap);
+    Table t;
+    t.keys = reinterpret_cast<int32_t *>(hub_smem);
+    t.lo = reinterpret_cast<unsigned *>(t.keys + kPartCap);
+    t.hi = t.lo + kPartCap;
+    t.list = nullptr;
+    int32_t *const keys = t.keys;
     __shared__ double sb[kHubPT / 32];
     __shared__ int32_t sm[kHubPT / 32];
     __shared__ int16_t taken[kPartCap / 2 + kHubPT];  // slots taken in this round, in the order taken
@@ -822,10 +827,7 @@ __global__ void __launch_bounds__(kHubPT, RMX_HUB_MINB) k_hub_eval(EvalArgs a, H
     const int32_t nu = (int32_t)p.tot[2];
     const int mask = kPartCap - 1;
     unsigned long long cands = 0;
-    for (int s = threadIdx.x; s < kPartCap; s += kHubPT) {
-        keys[s] = kEmpty;
-        vals[s] = 0;
-    }
+    table_clear(t, kPartCap, threadIdx.x, kHubPT);
     for (int64_t pidx = blockIdx.x; pidx < total; pidx += gridDim.x) {
         const int32_t j = p.punit[pidx];
         const int32_t u = a.list[h0 + j];
@@ -855,7 +857,7 @@ __global__ void __launch_bounds__(kHubPT, RMX_HUB_MINB) k_hub_eval(EvalArgs a, H
                     }
                     if (prev != kEmpty && prev != key) continue;  // unreachable: the table is never full
                     if (prev == kEmpty) taken[atomicAdd(&nfresh, 1)] = (int16_t)sl;
-                    atomic_add_fx(vals + sl, p.bfx[e]);
+                    table_add(t, sl, p.bfx[e]);
                 }
                 __syncthreads();
                 // at most kPartCap / 2 + kHubPT slots were taken (every thread checks the
@@ -866,16 +868,15 @@ __global__ void __launch_bounds__(kHubPT, RMX_HUB_MINB) k_hub_eval(EvalArgs a, H
                 for (int i = threadIdx.x; i < nt; i += kHubPT) {
                     const int s = taken[i];
                     const int32_t k = keys[s];
+                    const fx_t v = table_take(t, s);
                     if (!overfull && k != A) {
                         rc++;
-                        const double dl = candidate_delta(c, a.mrec[k], vals[s]);
+                        const double dl = candidate_delta(c, load_mod(a.mrec + k), v);
                         if (better(dl, k, rbest, rbm)) {
                             rbest = dl;
                             rbm = k;
                         }
                     }
-                    keys[s] = kEmpty;
-                    vals[s] = 0;
                 }
             }
             __syncthreads();
@@ -953,7 +954,7 @@ __global__ void k_hub_finish(EvalArgs a, HubPlan p) {
             const int32_t A = a.mod[u];
             const UnitCtx c = make_ctx<true>(a.attr[u], a.mrec[A], a.inst_sum_exit[a.uinst[u]], A,
                                        p.own[j]);
-            p.act[j] = (uint8_t)finish_unit(a, u, c, best, bm);
+            p.act[j] = (uint8_t)finish_unit(a, u, c, plogp(c.eu), plogp(c.eu + c.pu), best, bm, true);
             seen += unit_links(a, u);
             units++;
         }
@@ -1436,9 +1437,9 @@ int eval_tuning_generation() {
 }
 int64_t block_bin_max_degree() { return eval_tuning().large_max; }
 
-constexpr size_t kBlkSmem = (size_t)kBlkCap * (sizeof(fx_t) + sizeof(int32_t));
-constexpr size_t kMidSmem = (size_t)kMidCap * (sizeof(fx_t) + sizeof(int32_t));
-constexpr size_t kLrgSmem = (size_t)kLrgCap * (sizeof(fx_t) + sizeof(int32_t));
+constexpr size_t kBlkSmem = table_bytes(kBlkCap);
+constexpr size_t kMidSmem = table_bytes(kMidCap);
+constexpr size_t kLrgSmem = table_bytes(kLrgCap);
 
 // Blocks for `items` work items at per_block items a block, at most max_grid.
 static unsigned fit_grid(int64_t items, int64_t per_block, int64_t max_grid) {

@@ -126,6 +126,82 @@ __device__ __forceinline__ UnitCtx make_ctx(const Stat4 &ua, const ModRec &mA, d
     return c;
 }
 
+__device__ __forceinline__ ModRec load_mod(const ModRec *p) {
+    const double2 a = *reinterpret_cast<const double2 *>(&p->P), b = *reinterpret_cast<const double2 *>(&p->em);
+    ModRec r;
+    r.P = a.x;
+    r.TW = a.y;
+    r.em = b.x;
+    r.g = b.y;
+    r.t = p->t;
+    return r;
+}
+
+__device__ __forceinline__ Stat4 load_stat(const Stat4 *p) {
+    const longlong2 a = *reinterpret_cast<const longlong2 *>(&p->P);
+    const longlong2 b = *reinterpret_cast<const longlong2 *>(&p->D);
+    Stat4 r;
+    r.P = a.x;
+    r.TW = a.y;
+    r.D = b.x;
+    r.OUT = b.y;
+    return r;
+}
+
+// make_ctx for a group of W >= 8 lanes (gl = lane in the group): the six
+// logarithms of a unit (old module before and after, total exit, and the two of
+// the empty-module option) are taken by six lanes in one call instead of one
+// after another by all of them. newm: newmod_delta's unit terms.
+__device__ __forceinline__ UnitCtx make_ctx_lanes(int W, const Stat4 &ua, const ModRec &mA, double DA, double sum_exit, int32_t A,
+                                                  fx_t sA, int gl, double &new_exit, double &new_stay) {
+    const double2 tA = mA.t;
+    UnitCtx c;
+    c.pu = from_fx(ua.P);
+    c.tu = from_fx(ua.TW);
+    const double du = from_fx(ua.D);
+    c.eu = exit_flow(c.pu, c.tu, du, from_fx(ua.OUT));
+    c.cu = mix_flows(c.pu, du);
+    const double PA = mA.P, TWA = mA.TW;
+    c.eA = mA.em;
+    const double outA_inA = __fma_rn(mix_flows(PA - c.pu, DA - du), c.tu,
+                                     __fma_rn(c.cu, TWA - c.tu, __dmul_rn(kBeta, from_fx(sA))));
+    c.nexA = c.eA - c.eu + outA_inA;
+    c.sum_exit = sum_exit;
+    c.S0 = sum_exit + c.nexA - c.eA;
+    const double x = gl == 0   ? c.nexA
+                     : gl == 1 ? c.nexA + (PA - c.pu)
+                     : gl == 2 ? c.S0
+                     : gl == 3 ? sum_exit
+                     : gl == 4 ? c.eu
+                               : c.eu + c.pu;
+    const bool pos = x > 0.0;
+    const double lg = pos ? log(x) : 0.0;
+    const double pl = pos ? __dmul_rn(x, lg) : 0.0;
+    const double p0 = __shfl_sync(0xffffffffu, pl, 0, W), p1 = __shfl_sync(0xffffffffu, pl, 1, W),
+                 ps = __shfl_sync(0xffffffffu, pl, 3, W);
+    c.logS0 = __shfl_sync(0xffffffffu, lg, 2, W);
+    new_exit = __shfl_sync(0xffffffffu, pl, 4, W);
+    new_stay = __shfl_sync(0xffffffffu, pl, 5, W);
+    c.K = -ps - 2.0 * (p0 - tA.x) + (p1 - tA.y);
+    c.rS0 = c.S0 > 0.0 ? 1.0 / c.S0 : 0.0;
+    c.A = A;
+    return c;
+}
+
+// Lowest (change, module) over the warp. The change as an order-preserving
+// pair of 32-bit words, so that three hardware minimum reductions do it.
+__device__ __forceinline__ void warp_best(double &d, int32_t &m) {
+    const long long b = __double_as_longlong(d + 0.0);  // -0.0 counts as 0.0
+    const unsigned long long o =
+        b < 0 ? ~(unsigned long long)b : (unsigned long long)b ^ 0x8000000000000000ull;
+    const unsigned h = (unsigned)(o >> 32), l = (unsigned)o;
+    const unsigned mh = __reduce_min_sync(0xffffffffu, h);
+    const unsigned ml = __reduce_min_sync(0xffffffffu, h == mh ? l : 0xffffffffu);
+    m = __reduce_min_sync(0xffffffffu, h == mh && l == ml ? m : INT_MAX);
+    const unsigned long long r = ((unsigned long long)mh << 32) | ml;
+    d = __longlong_as_double(r & 0x8000000000000000ull ? (long long)(r ^ 0x8000000000000000ull) : (long long)~r);
+}
+
 __device__ __forceinline__ unsigned long long claim_key(uint32_t stamp, int32_t u) {
     return ((unsigned long long)stamp << 32) | (0xffffffffu - (uint32_t)u);
 }
