@@ -333,8 +333,9 @@ rmx_status rmx_sync(rmx_graph *g);
  * device's memory: the next handle or call of similar size (a cached
  * block is reused for requests of at least half its size) takes it without a
  * cudaMalloc / cudaFree pair, and an allocation that fails empties the cache
- * and retries. This frees every cached block (all devices); handles still open
- * are untouched. No reference counterpart (the reference holds no device
+ * and retries. This frees every cached block (all devices) and the 16 MB of
+ * pinned host memory through which large pageable inputs are copied; handles
+ * still open are untouched. No reference counterpart (the reference holds no device
  * memory). */
 rmx_status rmx_release_device_cache(void);
 

@@ -25,9 +25,9 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC,-O3,-Wall", "-diag-suppress", "177",
          *os.environ.get("RMX_NVCC_EXTRA", "").split()]
 CU = ["rmx_prims.cu", "rmx_flow.cu", "rmx_moves.cu", "rmx_stage.cu", "rmx_coarsen.cu", "rmx_convert.cu", "rmx_engine.cu", "rmx_adjoint.cu", "rmx_noalloc.cu"]
-CPP = ["rmx_io.cpp", "rmx_abi.cpp", "rmx_cli.cpp", "rmx_batch.cpp"]
-CUDA_CPP = {"rmx_abi.cpp", "rmx_batch.cpp"}
-HEADERS = ["rmx_common.cuh", "rmx_prims.cuh", "rmx_engine.cuh", "rmx_moves.cuh", "rmx_graph.hpp", "rmx_io.hpp", "rmx_batch.hpp"]
+CPP = ["rmx_io.cpp", "rmx_hostcopy.cpp", "rmx_abi.cpp", "rmx_cli.cpp", "rmx_batch.cpp"]
+CUDA_CPP = {"rmx_hostcopy.cpp", "rmx_abi.cpp", "rmx_batch.cpp"}
+HEADERS = ["rmx_common.cuh", "rmx_prims.cuh", "rmx_engine.cuh", "rmx_moves.cuh", "rmx_graph.hpp", "rmx_io.hpp", "rmx_hostcopy.hpp", "rmx_batch.hpp"]
 
 
 def _stale(target: Path, deps) -> bool:

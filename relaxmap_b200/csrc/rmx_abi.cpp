@@ -11,6 +11,7 @@
 
 #include "rmx_batch.hpp"
 #include "rmx_graph.hpp"
+#include "rmx_hostcopy.hpp"
 #include "rmx_io.hpp"
 
 namespace {
@@ -176,10 +177,10 @@ rmx_status rmx_graph_links(const rmx_graph *g, int64_t *off, int32_t *dst, doubl
     return guard([&] {
         need(g, "graph");
         cudaStream_t s = g->stream;
-        if (off) RMX_CUDA(cudaMemcpyAsync(off, g->out_off, sizeof(int64_t) * (g->N + 1), cudaMemcpyDeviceToHost, s));
-        if (dst && g->E) RMX_CUDA(cudaMemcpyAsync(dst, g->out_dst, sizeof(int32_t) * g->E, cudaMemcpyDeviceToHost, s));
-        if (w && g->E) RMX_CUDA(cudaMemcpyAsync(w, g->out_w0, sizeof(double) * g->E, cudaMemcpyDeviceToHost, s));
-        if (teleport) RMX_CUDA(cudaMemcpyAsync(teleport, g->tw, sizeof(double) * g->N, cudaMemcpyDeviceToHost, s));
+        if (off) rmx::download(off, g->out_off, sizeof(int64_t) * (g->N + 1), s);
+        if (dst && g->E) rmx::download(dst, g->out_dst, sizeof(int32_t) * g->E, s);
+        if (w && g->E) rmx::download(w, g->out_w0, sizeof(double) * g->E, s);
+        if (teleport) rmx::download(teleport, g->tw, sizeof(double) * g->N, s);
         RMX_CUDA(cudaStreamSynchronize(s));
     });
 }
@@ -190,14 +191,14 @@ rmx_status rmx_initiate(rmx_graph *g, double *p, double *f, double *exitpr, uint
         need(g, "graph");
         g->initiate();
         cudaStream_t s = g->stream;
-        if (p) RMX_CUDA(cudaMemcpyAsync(p, g->p, sizeof(double) * g->N, cudaMemcpyDeviceToHost, s));
-        if (f && g->E) RMX_CUDA(cudaMemcpyAsync(f, g->out_f, sizeof(double) * g->E, cudaMemcpyDeviceToHost, s));
-        if (dangling) RMX_CUDA(cudaMemcpyAsync(dangling, g->dangling, g->N, cudaMemcpyDeviceToHost, s));
+        if (p) rmx::download(p, g->p, sizeof(double) * g->N, s);
+        if (f && g->E) rmx::download(f, g->out_f, sizeof(double) * g->E, s);
+        if (dangling) rmx::download(dangling, g->dangling, g->N, s);
         if (exitpr) {
             size_t mk = g->scratch.mark();
             double *ex = g->scratch.alloc<double>(g->N);
             rmx::singleton_exits(g->N, g->out_off, g->out_f, g->p, g->tw, g->dangling, ex, s);
-            RMX_CUDA(cudaMemcpyAsync(exitpr, ex, sizeof(double) * g->N, cudaMemcpyDeviceToHost, s));
+            rmx::download(exitpr, ex, sizeof(double) * g->N, s);
             RMX_CUDA(cudaStreamSynchronize(s));
             g->scratch.release(mk);
         }
@@ -496,7 +497,10 @@ rmx_status rmx_set_tuning(const rmx_tuning *t) {
 }
 
 rmx_status rmx_release_device_cache(void) {
-    return guard([&] { rmx::release_device_cache(); });
+    return guard([&] {
+        rmx::release_device_cache();
+        rmx::release_upload_ring();
+    });
 }
 
 }  // extern "C"

@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "rmx_graph.hpp"
+#include "rmx_hostcopy.hpp"
 
 namespace cg = cooperative_groups;
 
@@ -468,7 +469,7 @@ void rmx_graph::adjoint(const int32_t *part_host, double tau, double *L_out, dou
     const double plq = Q > 0.0 ? Q * std::log(Q) : 0.0;
     const double L = plq - 2.0 * sq + sqp - from_fxl(s0h);
     if (L_out) *L_out = L;
-    if (p_out) RMX_CUDA(cudaMemcpyAsync(p_out, pa, sizeof(double) * N, cudaMemcpyDeviceToHost, stream));
+    if (p_out) download(p_out, pa, sizeof(double) * N, stream);
     if (grad_out || dL_dtau) {
         const double beta = 1.0 - tau;
         k_adj_mod2<<<G, kAdjT, 0, stream>>>(N, mst, q, Q > 0.0 ? std::log(Q) : 0.0, gm, hm, parts);
@@ -508,7 +509,7 @@ void rmx_graph::adjoint(const int32_t *part_host, double tau, double *L_out, dou
                 k_adj_grad<<<blocks_for((int64_t)N * 32, 256, num_sms() * 32), 256, 0, stream>>>(
                     N, out_off, out_dst, out_w0, rowsum, part, pa, gm, lam, beta, grad);
                 RMX_LAUNCHED();
-                RMX_CUDA(cudaMemcpyAsync(grad_out, grad, sizeof(double) * E, cudaMemcpyDeviceToHost, stream));
+                download(grad_out, grad, sizeof(double) * E, stream);
             }
         }
         if (dL_dtau) {

@@ -12,6 +12,7 @@
 #include <cstring>
 
 #include "rmx_graph.hpp"
+#include "rmx_hostcopy.hpp"
 #include "rmx_io.hpp"
 
 using namespace rmx;
@@ -467,9 +468,9 @@ void rmx_graph::create(const int32_t *src, const int32_t *dst, const double *w, 
     if (n_edges >= (int64_t(1) << 31)) throw std::invalid_argument("more than 2^31-1 input edges");
     const bool repl = u && u->n_canon > 0;  // edges describe the canonical copies only
     const int32_t n_in = repl ? u->n_canon : n;
-    {  // endpoints checked on host threads (one below 4M edges), before any device work
+    {  // endpoints checked on host threads (one below 2^20 edges), before any device work
         const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-        const int T = (int)std::min<int64_t>(std::min(hw, 16u), std::max<int64_t>(1, n_edges >> 22));
+        const int T = (int)std::min<int64_t>(std::min(hw, 16u), std::max<int64_t>(1, n_edges >> 19));
         std::vector<uint8_t> bad(std::max(T, 1), 0);
         rmx::run_parallel(T, [&](int t) {
             const int64_t e0 = n_edges * t / T, e1 = n_edges * (t + 1) / T;
@@ -507,10 +508,10 @@ void rmx_graph::create(const int32_t *src, const int32_t *dst, const double *w, 
     int32_t *d_src = scratch.alloc<int32_t>(Ein), *d_dst = scratch.alloc<int32_t>(Ein);
     double *d_w = scratch.alloc<double>(Ein);
     if (n_edges > 0) {
-        RMX_CUDA(cudaMemcpyAsync(d_src, src, sizeof(int32_t) * n_edges, cudaMemcpyHostToDevice, stream));
-        RMX_CUDA(cudaMemcpyAsync(d_dst, dst, sizeof(int32_t) * n_edges, cudaMemcpyHostToDevice, stream));
+        upload(d_src, src, sizeof(int32_t) * n_edges, stream);
+        upload(d_dst, dst, sizeof(int32_t) * n_edges, stream);
         if (w)
-            RMX_CUDA(cudaMemcpyAsync(d_w, w, sizeof(double) * n_edges, cudaMemcpyHostToDevice, stream));
+            upload(d_w, w, sizeof(double) * n_edges, stream);
         else {
             k_fill<<<blocks_for(n_edges, 256, 4096), 256, 0, stream>>>(d_w, n_edges, 1.0);
             RMX_LAUNCHED();
@@ -1484,9 +1485,7 @@ double rmx_graph::optimize(const rmx_opts &o, int32_t *part_out, int32_t *n_modu
         }
     }
     step_bits = best_steps;
-    if (part_out)
-        RMX_CUDA(cudaMemcpyAsync(part_out, opt.attempts > 1 ? best_part : nmod, sizeof(int32_t) * N,
-                                 cudaMemcpyDeviceToHost, stream));
+    if (part_out) download(part_out, opt.attempts > 1 ? best_part : nmod, sizeof(int32_t) * N, stream);
     RMX_CUDA(cudaEventRecord(t1, stream));
     RMX_CUDA(cudaEventSynchronize(t1));
     float ms = 0;
