@@ -230,11 +230,11 @@ void rows_of_links(int32_t n, const int64_t *off, int32_t *src, cudaStream_t s) 
     RMX_LAUNCHED();
 }
 
-// glinks[g]: links of g's members (the capacity of g's range).
+// glinks[g]: links of g's members (the capacity of g's range). Rows without a group (-1) count nowhere.
 __global__ void k_agg_count(int32_t n, const int64_t *off, const int32_t *group, unsigned long long *glinks) {
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
         const int64_t d = off[r + 1] - off[r];
-        if (d) atomicAdd(glinks + group[r], (unsigned long long)d);
+        if (d && group[r] >= 0) atomicAdd(glinks + group[r], (unsigned long long)d);
     }
 }
 
@@ -252,9 +252,11 @@ __global__ void k_agg_gather(int64_t m, const int32_t *src, const int32_t *dst, 
         fx_t q = 0;
         if (e < m) {
             g = __ldg(group + __ldcs(src + e));  // links streamed, group ids kept in L2
-            b = __ldg(group + __ldcs(dst + e));
-            q = __ldcs(fx + e);
-            if (b == g) g = -1;  // links inside a group are not kept
+            if (g >= 0) {
+                b = __ldg(group + __ldcs(dst + e));
+                q = __ldcs(fx + e);
+                if (b == g) g = -1;  // links inside a group are not kept
+            }
         }
         const unsigned peers = __match_any_sync(kFullMask, g);
         const int leader = __ffs(peers) - 1;

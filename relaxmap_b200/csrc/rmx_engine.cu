@@ -62,6 +62,16 @@ __global__ void k_group_of_nodes(int32_t n, const int32_t *mod, const int64_t *s
         node_sn[v] = (int32_t)snid[mod[v]];
 }
 
+// The groups whose links are to be summed: units of instances that have stopped
+// get none (-1). They keep their modules, are not evaluated again and take part
+// in no later conversion of this superstep, and every superstep starts from the
+// node links, so their links are never needed.
+__global__ void k_group_live(int32_t n, const int32_t *mod, const int64_t *snid, const int32_t *inst,
+                             const uint8_t *live, int32_t *group) {
+    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x)
+        group[v] = live[inst[v]] ? (int32_t)snid[mod[v]] : -1;
+}
+
 __global__ void k_project(int32_t n, const int32_t *node_sn, const int32_t *sn_mod, int32_t *nmod) {
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x)
         nmod[v] = sn_mod[node_sn[v]];
@@ -69,10 +79,16 @@ __global__ void k_project(int32_t n, const int32_t *node_sn, const int32_t *sn_m
 
 // Intra-module links for the coarse-tune sub-networks (generate_network_from_module,
 // OmpRelaxmap.cpp:664-684): per row, the links whose other end shares the module.
-__global__ void k_intra_count(int32_t n, const int64_t *off, const int32_t *nbr, const int32_t *mod, int64_t *cnt) {
+// live (may be null): rows of instances that have stopped (inst) have none.
+__global__ void k_intra_count(int32_t n, const int64_t *off, const int32_t *nbr, const int32_t *mod, int64_t *cnt,
+                              const int32_t *inst, const uint8_t *live) {
     const int lane = threadIdx.x & 31;
     const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t u = gw; u < n; u += nw) {
+        if (live && !live[inst[u]]) {
+            if (lane == 0) cnt[u] = 0;
+            continue;
+        }
         const int32_t m = mod[u];
         int c = 0;
         for (int64_t e = off[u] + lane; e < off[u + 1]; e += 32) c += mod[nbr[e]] == m;
@@ -83,7 +99,8 @@ __global__ void k_intra_count(int32_t n, const int64_t *off, const int32_t *nbr,
 }
 
 __global__ void k_intra_fill(int32_t n, const int64_t *off, const int32_t *nbr, const fx_t *fx, const int32_t *mod,
-                             const int64_t *noff, int32_t *nnbr, fx_t *nfx, fx_t *row_sum) {
+                             const int64_t *noff, int32_t *nnbr, fx_t *nfx, fx_t *row_sum, const int32_t *inst,
+                             const uint8_t *live) {
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
     const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -91,9 +108,10 @@ __global__ void k_intra_fill(int32_t n, const int64_t *off, const int32_t *nbr, 
         const int32_t m = mod[u];
         int64_t pos = noff[u];
         fx_t sum = 0;
-        for (int64_t base = off[u]; base < off[u + 1]; base += 32) {
+        const int64_t end = !live || live[inst[u]] ? off[u + 1] : off[u];
+        for (int64_t base = off[u]; base < end; base += 32) {
             const int64_t e = base + lane;
-            const bool keep = e < off[u + 1] && mod[nbr[e]] == m;
+            const bool keep = e < end && mod[nbr[e]] == m;
             const unsigned bal = __ballot_sync(kFull, keep);
             if (keep) {
                 const int64_t q = pos + __popc(bal & lt);
@@ -692,6 +710,8 @@ void rmx_graph::alloc_engine() {
     stage_seed = perm.alloc<uint32_t>(8);
     stage_sweeping = perm.alloc<uint8_t>(std::max(K, 1));
     stage_oldL = perm.alloc<double>(std::max(K, 1));
+    live = perm.alloc<uint8_t>(std::max(K, 1));
+    RMX_CUDA(cudaMemsetAsync(live, 1, (size_t)std::max(K, 1), stream));
     RMX_CUDA(cudaMemsetAsync(work.stamp, 0, sizeof(uint32_t) * n, stream));
     RMX_CUDA(cudaMemsetAsync(work.claim, 0, sizeof(unsigned long long) * n, stream));
     RMX_CUDA(cudaMemsetAsync(work.next_active, 0, n, stream));
@@ -1200,7 +1220,13 @@ void rmx_graph::convert_to_supernodes(bool from_sn) {
         N, mods.count, snid, mods.stat, K > 1 ? mods.inst : nullptr, dst.mod, dst.attr, dst.nnodes, dst.inst);
     RMX_LAUNCHED();
     int32_t *group = nullptr;
-    if (from_sn) {
+    if (K > 1) {
+        const int32_t n = from_sn ? src.n : N;
+        group = scratch.alloc<int32_t>(std::max(n, 1));
+        k_group_live<<<blocks_for(n, 256, num_sms() * 32), 256, 0, stream>>>(
+            n, from_sn ? src.mod : nmod, snid, from_sn ? src.inst : node_inst, live, group);
+        RMX_LAUNCHED();
+    } else if (from_sn) {
         group = scratch.alloc<int32_t>(std::max(src.n, 1));
         k_group_of_nodes<<<blocks_for(src.n, 256, num_sms() * 32), 256, 0, stream>>>(src.n, src.mod, snid, group);
         RMX_LAUNCHED();
@@ -1214,7 +1240,7 @@ void rmx_graph::convert_to_supernodes(bool from_sn) {
                                 dst.out_dst, dst.out_fx, dst.out_src, dst.in_off, dst.in_src, dst.in_fx, nullptr,
                                 agg_arena, agg_tab, agg_cap, scratch, stream, &work);
     else
-        dst.m = aggregate_links(N, out_off, out_dst, out_fx, node_lv.out_src, node_sn, dst.n, dst.out_off, dst.out_dst,
+        dst.m = aggregate_links(N, out_off, out_dst, out_fx, node_lv.out_src, group ? group : node_sn, dst.n, dst.out_off, dst.out_dst,
                                 dst.out_fx, dst.out_src, dst.in_off, dst.in_src, dst.in_fx, nullptr, agg_arena, agg_tab,
                                 agg_cap, scratch, stream, &work);
     scratch.release(mk);
@@ -1255,18 +1281,19 @@ void rmx_graph::generate_sub_modules() {
     const unsigned GW = blocks_for((int64_t)N * 32, 256, num_sms() * 32);
     RMX_CUDA(cudaMemsetAsync(cnt_out + N, 0, sizeof(int64_t), stream));
     RMX_CUDA(cudaMemsetAsync(cnt_in + N, 0, sizeof(int64_t), stream));
-    k_intra_count<<<GW, 256, 0, stream>>>(N, out_off, out_dst, nmod, cnt_out);
+    const uint8_t *const lv = K > 1 ? inst1.active : nullptr;  // the instances of the next superstep
+    k_intra_count<<<GW, 256, 0, stream>>>(N, out_off, out_dst, nmod, cnt_out, node_inst, lv);
     RMX_LAUNCHED();
-    k_intra_count<<<GW, 256, 0, stream>>>(N, in_off, in_src, nmod, cnt_in);
+    k_intra_count<<<GW, 256, 0, stream>>>(N, in_off, in_src, nmod, cnt_in, node_inst, lv);
     RMX_LAUNCHED();
     scan_exclusive(cnt_out, sub_lv.out_off, N + 1, nullptr, scratch, stream);
     scan_exclusive(cnt_in, sub_lv.in_off, N + 1, nullptr, scratch, stream);
     fx_t *intra_out = reinterpret_cast<fx_t *>(cnt_out);  // counts are consumed by the scans above
     k_intra_fill<<<GW, 256, 0, stream>>>(N, out_off, out_dst, out_fx, nmod, sub_lv.out_off, sub_lv.out_dst,
-                                         sub_lv.out_fx, intra_out);
+                                         sub_lv.out_fx, intra_out, node_inst, lv);
     RMX_LAUNCHED();
     k_intra_fill<<<GW, 256, 0, stream>>>(N, in_off, in_src, in_fx, nmod, sub_lv.in_off, sub_lv.in_src, sub_lv.in_fx,
-                                         nullptr);
+                                         nullptr, node_inst, lv);
     RMX_LAUNCHED();
     k_sub_attr<<<blocks_for(N, 256, num_sms() * 32), 256, 0, stream>>>(N, nattr, intra_out, sub_lv.attr);
     RMX_LAUNCHED();
@@ -1347,7 +1374,13 @@ void rmx_graph::generate_sub_modules() {
     RMX_LAUNCHED();
     {
         fx_t *rowsum = scratch.alloc<fx_t>(std::max<int64_t>(nsn, 1));
-        sl.m = aggregate_links(N, out_off, out_dst, out_fx, node_lv.out_src, node_sn, sl.n, sl.out_off, sl.out_dst,
+        int32_t *group = node_sn;
+        if (K > 1) {
+            group = scratch.alloc<int32_t>(N);
+            k_group_live<<<blocks_for(N, 256, num_sms() * 32), 256, 0, stream>>>(N, submod, snid, node_inst, lv, group);
+            RMX_LAUNCHED();
+        }
+        sl.m = aggregate_links(N, out_off, out_dst, out_fx, node_lv.out_src, group, sl.n, sl.out_off, sl.out_dst,
                                sl.out_fx, sl.out_src, sl.in_off, sl.in_src, sl.in_fx, rowsum, agg_arena, agg_tab, agg_cap,
                                scratch, stream, &work);
         k_sn_set_out<<<blocks_for(nsn, 256, num_sms() * 32), 256, 0, stream>>>(sl.n, rowsum, sl.attr);
@@ -1372,6 +1405,7 @@ void rmx_graph::stage(bool fine, std::vector<double> &L, const std::vector<uint8
     bool from_sn = !fine;  // after node sweeps the first conversion reads the node links
     do {
         oldL = L;
+        if (K > 1) RMX_CUDA(cudaMemcpyAsync(live, act.data(), (size_t)K, cudaMemcpyHostToDevice, stream));
         convert_to_supernodes(from_sn);
         from_sn = true;
         stage_sweeps(sn(), true, L, act);

@@ -297,7 +297,8 @@ int64_t coarsen_links(int32_t n, const int64_t *out_off, const int32_t *out_dst,
 // fixed-point sums only, rows and columns in no particular order. src: the
 // row of every input link (CSR order); g_out_src receives the row (group) of
 // every output link. rowsum (may be NULL) receives each group's total
-// out-flow. gtab / gtab_cap: a global table in gtab_arena, grown on demand for
+// out-flow. Rows of group -1 are left out with all their links, which must
+// lead to rows of group -1 too. gtab / gtab_cap: a global table in gtab_arena, grown on demand for
 // groups too large for shared memory. W (may be NULL): auxiliary streams and
 // events on which the size bins run concurrently.
 int64_t aggregate_links(int32_t n, const int64_t *off, const int32_t *dst, const fx_t *fx, const int32_t *src,

@@ -122,6 +122,7 @@ struct rmx_graph {
     // graph-attempt copies, node ranges inst_noff[k]..inst_noff[k+1]
     int32_t K = 1;
     int32_t *node_inst = nullptr;       // device: instance of every node (zeros when K == 1)
+    uint8_t *live = nullptr;            // device: instances whose links the next conversion sums (K > 1)
     std::vector<int64_t> inst_noff;     // host, K + 1
     std::vector<int32_t> inst_canon;    // host: the copy whose flow instance k shares (itself if first)
     std::vector<double> L0v;            // initial code length per instance
