@@ -839,7 +839,7 @@ int rmx_graph::union_flows() {
     RMX_CUDA(cudaMemcpyAsync(d_comp, comp.data(), sizeof(int64_t) * comp.size(), cudaMemcpyHostToDevice, stream));
     RMX_CUDA(cudaMemcpyAsync(d_noff, inst_noff.data(), sizeof(int64_t) * (K + 1), cudaMemcpyHostToDevice, stream));
     RMX_CUDA(cudaMemcpyAsync(d_canon, inst_canon.data(), sizeof(int32_t) * K, cudaMemcpyHostToDevice, stream));
-    const int it = power_iteration_components(N, nc, d_comp, node_inst, d_noff, d_canon, in_off, in_src, in_w, tw,
+    const int it = power_iteration_components(N, nc, comp.data(), d_comp, node_inst, d_noff, d_canon, in_off, in_src, in_w, tw,
                                               dangling, p, scratch, stream, spmv_vec);
     scratch.release(mk);
     return it;

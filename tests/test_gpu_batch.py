@@ -117,3 +117,23 @@ def test_batch_captured_loops_match_host_loops(built_lib, capfd):
     np.testing.assert_array_equal(a["best_attempt"], b["best_attempt"])
     for pa, pb in zip(a["part"], b["part"]):
         np.testing.assert_array_equal(pa, pb)
+
+
+@pytest.mark.parametrize("attempts", [1, 3])
+def test_union_flow_of_uneven_graphs(built_lib, attempts):
+    """Graphs whose sizes leave part of a row group, of a block and of a warp's run over, with and
+    without dangling nodes: each returned code length is the single-graph one of its partition."""
+    from relaxmap_b200 import Batch, Graph
+    rng = np.random.default_rng(3)
+    graphs = []
+    for n in (2, 3, 31, 33, 255, 256, 257, 2049, 6001):
+        m = 5 * n
+        src, dst = rng.integers(0, max(1, n - n // 7), m), rng.integers(0, n, m)
+        src[0], dst[0] = 0, n - 1
+        key = np.unique((src * np.int64(n) + dst)[src != dst])
+        graphs.append((n, (key // n).astype(np.int32), (key % n).astype(np.int32), rng.uniform(1, 5, len(key))))
+    with Batch(graphs) as b:
+        r = b.optimize(seed=3, attempts=attempts)
+    for (n, src, dst, w), part, L in zip(graphs, r["part"], r["L"]):
+        with Graph.from_edges(src, dst, w, n=n) as g:
+            assert abs(g.codelength(part) - L) <= 1e-10
