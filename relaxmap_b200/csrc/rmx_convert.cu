@@ -306,30 +306,49 @@ __global__ void __launch_bounds__(kCvT, 1) k_convert(const __grid_constant__ Con
         if (g < ng) a.gloff[g] = base + x - c;
     }
     grid.sync();
-    // links between groups, gathered into the source group's room
-    for (int64_t e0 = gw * 32; e0 < a.m; e0 += nw * 32) {
-        const int64_t e = e0 + lane;
-        int32_t g = -1, b = -1;
-        fx_t q = 0;
-        if (e < a.m) {
-            g = group[a.src[e]];
-            b = group[a.dst[e]];
-            q = a.fx[e];
-            if (b == g) g = -1;
+    // links between groups, gathered into the source group's room, four per lane at a time
+    for (int64_t e0 = gw * 32; e0 < a.m; e0 += nw * 32 * kCvIlp) {
+        int32_t g[kCvIlp], b[kCvIlp];
+        fx_t q[kCvIlp];
+#pragma unroll
+        for (int k = 0; k < kCvIlp; k++) {
+            const int64_t e = e0 + k * nw * 32 + lane;
+            g[k] = b[k] = 0;
+            q[k] = 0;
+            if (e0 + k * nw * 32 < a.m) {  // warp-uniform; lanes past the links read the last one
+                const int64_t c = min(e, a.m - 1);
+                g[k] = a.src[c];
+                b[k] = a.dst[c];
+                q[k] = a.fx[c];
+            }
         }
-        // lanes of a run of links with the same source group (rows follow one another) take their places together
-        const int32_t before = __shfl_up_sync(kFull, g, 1);
-        const unsigned heads = __ballot_sync(kFull, lane == 0 || before != g);
-        const int head = 31 - __clz(heads & (kFull >> (31 - lane)));
-        const unsigned after = lane == 31 ? 0u : heads & (kFull << (lane + 1));
-        const int end = after ? __ffs(after) - 1 : 32;
-        unsigned base = 0;
-        if (g >= 0 && lane == head) base = atomicAdd(a.gcross + g, (unsigned)(end - head));
-        base = __shfl_sync(kFull, base, head);
-        if (g >= 0) {
-            const unsigned p = a.gloff[g] + base + (unsigned)(lane - head);
-            a.sk[p] = b;
-            a.sq[p] = q;
+#pragma unroll
+        for (int k = 0; k < kCvIlp; k++) {
+            g[k] = group[g[k]];
+            b[k] = group[b[k]];
+        }
+        unsigned base[kCvIlp];
+        int head[kCvIlp];
+#pragma unroll
+        for (int k = 0; k < kCvIlp; k++) {
+            if (e0 + k * nw * 32 + lane >= a.m || b[k] == g[k]) g[k] = -1;
+            // lanes of a run of links with the same source group (rows follow one another) take their places together
+            const int32_t before = __shfl_up_sync(kFull, g[k], 1);
+            const unsigned heads = __ballot_sync(kFull, lane == 0 || before != g[k]);
+            head[k] = 31 - __clz(heads & (kFull >> (31 - lane)));
+            const unsigned after = lane == 31 ? 0u : heads & (kFull << (lane + 1));
+            const int end = after ? __ffs(after) - 1 : 32;
+            base[k] = 0;
+            if (g[k] >= 0 && lane == head[k]) base[k] = atomicAdd(a.gcross + g[k], (unsigned)(end - head[k]));
+        }
+#pragma unroll
+        for (int k = 0; k < kCvIlp; k++) {
+            base[k] = __shfl_sync(kFull, base[k], head[k]);
+            if (g[k] >= 0) {
+                const unsigned p = a.gloff[g[k]] + base[k] + (unsigned)(lane - head[k]);
+                a.sk[p] = b[k];
+                a.sq[p] = q[k];
+            }
         }
     }
     grid.sync();
@@ -437,21 +456,46 @@ __global__ void __launch_bounds__(kCvT, 1) k_convert(const __grid_constant__ Con
         }
     }
     grid.sync();
-    // rows, eight lanes each, and their entries in the columns
+    // rows, eight lanes each (the whole warp for rows of more than 64 entries), and their entries in the columns
+    auto put = [&](int32_t g, unsigned from, int64_t to, unsigned len, int r, int width) {
+        for (unsigned j0 = 0; j0 < len; j0 += kCvIlp * width) {
+            int32_t b[kCvIlp];
+            fx_t q[kCvIlp];
+            int64_t p[kCvIlp];
+#pragma unroll
+            for (int k = 0; k < kCvIlp; k++) {
+                const unsigned j = j0 + k * width + r;
+                b[k] = -1;
+                if (j < len) {
+                    b[k] = a.rk[from + j];
+                    q[k] = a.rq[from + j];
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < kCvIlp; k++)
+                if (b[k] >= 0) p[k] = a.in_off[b[k]] + atomicAdd(a.colfill + b[k], 1u);
+#pragma unroll
+            for (int k = 0; k < kCvIlp; k++)
+                if (b[k] >= 0) {
+                    const int64_t j = to + j0 + k * width + r;
+                    a.out_dst[j] = b[k];
+                    a.out_fx[j] = q[k];
+                    a.out_src[j] = g;
+                    a.in_src[p[k]] = g;
+                    a.in_fx[p[k]] = q[k];
+                }
+        }
+    };
     for (int64_t r0 = gw * 4; r0 < ng; r0 += nw * 4) {
         const int64_t g = r0 + (lane >> 3);
-        if (g >= ng) continue;
-        const unsigned from = a.gloff[g], len = a.rowlen[g];
-        const int64_t to = a.out_off[g];
-        for (unsigned j = lane & 7; j < len; j += 8) {
-            const int32_t b = a.rk[from + j];
-            const fx_t q = a.rq[from + j];
-            a.out_dst[to + j] = b;
-            a.out_fx[to + j] = q;
-            a.out_src[to + j] = (int32_t)g;
-            const int64_t p = a.in_off[b] + atomicAdd(a.colfill + b, 1u);
-            a.in_src[p] = (int32_t)g;
-            a.in_fx[p] = q;
+        const unsigned from = g < ng ? a.gloff[g] : 0u, len = g < ng ? a.rowlen[g] : 0u;
+        const int64_t to = g < ng ? a.out_off[g] : 0;
+        if (len <= 64) put((int32_t)g, from, to, len, lane & 7, 8);
+        __syncwarp();
+        for (int k = 0; k < 4; k++) {
+            const unsigned l = __shfl_sync(kFull, len, 8 * k);
+            if (l > 64)
+                put((int32_t)(r0 + k), __shfl_sync(kFull, from, 8 * k), __shfl_sync(kFull, to, 8 * k), l, lane, 32);
         }
     }
 }

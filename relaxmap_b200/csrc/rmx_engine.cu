@@ -21,15 +21,13 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 const double kLn2 = std::log(2.0);
-// Largest source level converted in one launch. On the levels of the planted
-// graph of 20,011 nodes (209,114 links) it takes 0.12 ms against 0.26 ms by
-// separate kernels, on those of 150,001 nodes (2.5 to 2.9 million links) 0.45
-// against 0.44 ms, on those of 1M nodes (19 million) 1.6 against 1.2 ms: there
-// 16 warps per SM keep fewer links in flight than the separate kernels.
-#ifndef RMX_CONVERT_MAX
-#define RMX_CONVERT_MAX (1 << 20)
-#endif
-constexpr int64_t kConvertMaxLinks = RMX_CONVERT_MAX;
+// Largest source level converted in one launch. All conversions of a run took,
+// by separate kernels and in one launch: planted graphs of 60,013 nodes (1.1
+// million links) 8.0 and 4.2 ms, 150,001 nodes (2.9 million) 11.1 and 8.6 ms,
+// 400,001 nodes (7.6 million) 40.6 and 37.9 ms, 1M nodes (19 million) 51.5 and
+// 54.3 ms: there 16 warps per SM keep fewer links in flight than the separate
+// kernels do.
+constexpr int64_t kConvertMaxLinks = 1 << 23;
 
 __global__ void k_fill(double *a, int64_t n, double v) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
