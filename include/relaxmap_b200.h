@@ -195,6 +195,15 @@ rmx_status rmx_coarsen_engine(rmx_graph *g, const int32_t *part, const int32_t *
                               int64_t *n_sn_links, int32_t *sn_of_mod, int64_t *out_off, int32_t *out_dst,
                               int64_t *out_fx, int64_t *in_off, int32_t *in_src, int64_t *in_fx, int64_t *sn_stat);
 
+/* The coarse-tune level of a given partition (the sub-networks of
+ * generate_sub_modules, OmpRelaxmap.cpp:502-638): every node's links to nodes
+ * of its own module, flows fixed point as above, and out_sum[N], each node's
+ * sum over its out-links. Rows come in no particular order. Buffers are sized
+ * N (+1 for offsets) and E by the caller; the handle's partition state is
+ * overwritten. */
+rmx_status rmx_sub_level(rmx_graph *g, const int32_t *part, int64_t *n_links, int64_t *out_off, int32_t *out_dst,
+                         int64_t *out_fx, int64_t *in_off, int32_t *in_src, int64_t *in_fx, int64_t *out_sum);
+
 /* The move decision of every super-node against a fixed snapshot (the
  * evaluation phase of Network::parallelMoveSuperNodes, Module.cpp:2198-2313,
  * and prioritize_parallelMoveSPnodes, :2555-2670): the super-node level of
@@ -306,7 +315,7 @@ typedef struct rmx_tuning {
     int32_t eval_mid_grid;    /* mid bin (default 8) */
     int32_t eval_block_grid;  /* block bin (default 4) */
     int32_t eval_large_grid;  /* large bin (default 2) */
-    int32_t eval_warp_grid;   /* warp bin (default 3) */
+    int32_t eval_warp_grid;   /* warp bin (default 4) */
     int32_t eval_reg_grid;    /* register bins (default 8) */
     int32_t warp_max_degree;  /* default 128 */
     int32_t mid_max_degree;   /* default 512 */

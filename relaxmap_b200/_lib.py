@@ -23,7 +23,7 @@ KERNELS = ["spmv", "eval", "commit", "coarsen", "codelen", "other", "adjoint"]
 EXPORTS = ["rmx_last_error", "rmx_version", "rmx_opts_default", "rmx_graph_create", "rmx_graph_load_file",
            "rmx_parse_file",
            "rmx_graph_destroy", "rmx_graph_info", "rmx_graph_links", "rmx_initiate", "rmx_codelength",
-           "rmx_coarsen", "rmx_evaluate_moves", "rmx_coarsen_engine", "rmx_evaluate_sn_moves", "rmx_optimize", "rmx_superstep_codelengths", "rmx_write_outputs",
+           "rmx_coarsen", "rmx_evaluate_moves", "rmx_coarsen_engine", "rmx_sub_level", "rmx_evaluate_sn_moves", "rmx_optimize", "rmx_superstep_codelengths", "rmx_write_outputs",
            "rmx_set_profiling", "rmx_get_profile", "rmx_graph_stream", "rmx_sync", "rmx_cli_main",
            "rmx_steady_state_noalloc", "rmx_noalloc_last_error", "rmx_adjoint_forward", "rmx_adjoint_backward",
            "rmx_batch_create", "rmx_batch_set_wave", "rmx_batch_optimize", "rmx_batch_info", "rmx_batch_destroy",
@@ -238,6 +238,19 @@ class Graph:
         k, s = nl.value, nsn.value
         return dict(n_sn=s, sn_of_mod=snm, out_off=oo[:s + 1], out_dst=od[:k], out_fx=of[:k], in_off=io[:s + 1],
                     in_src=is_[:k], in_fx=if_[:k], sn_stat=st[:s])
+
+    def sub_level(self, part) -> dict:
+        """The coarse-tune level of part: every node's links inside its module
+        (fixed-point flows, value * 2^62), rows in the engine's order."""
+        part = np.ascontiguousarray(part, dtype=np.int32)
+        n, m, nl = self.n, max(self.n_links, 1), C.c_int64()
+        oo, od, of = np.zeros(n + 1, dtype=np.int64), np.zeros(m, dtype=np.int32), np.zeros(m, dtype=np.int64)
+        io, is_, if_ = np.zeros(n + 1, dtype=np.int64), np.zeros(m, dtype=np.int32), np.zeros(m, dtype=np.int64)
+        sums = np.zeros(n, dtype=np.int64)
+        _check(lib().rmx_sub_level(self._h, _p(part), C.byref(nl), _p(oo), _p(od), _p(of), _p(io), _p(is_), _p(if_),
+                                   _p(sums)))
+        k = nl.value
+        return dict(out_off=oo, out_dst=od[:k], out_fx=of[:k], in_off=io, in_src=is_[:k], in_fx=if_[:k], out_sum=sums)
 
     def evaluate_sn_moves(self, part, sn_part, allow_new=None):
         """Move decisions of the super-nodes of part placed in modules sn_part."""

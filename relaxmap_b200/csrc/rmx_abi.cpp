@@ -330,6 +330,20 @@ rmx_status rmx_coarsen_engine(rmx_graph *g, const int32_t *part, const int32_t *
     });
 }
 
+rmx_status rmx_sub_level(rmx_graph *g, const int32_t *part, int64_t *n_links, int64_t *out_off, int32_t *out_dst,
+                         int64_t *out_fx, int64_t *in_off, int32_t *in_src, int64_t *in_fx, int64_t *out_sum) {
+    return guard([&] {
+        need(g, "graph");
+        need(part, "part");
+        for (const void *p : {(const void *)n_links, (const void *)out_off, (const void *)out_dst, (const void *)out_fx,
+                              (const void *)in_off, (const void *)in_src, (const void *)in_fx, (const void *)out_sum})
+            need(p, "output");
+        using fxp = rmx::fx_t *;
+        g->sub_level_hook(part, n_links, out_off, out_dst, reinterpret_cast<fxp>(out_fx), in_off, in_src,
+                          reinterpret_cast<fxp>(in_fx), reinterpret_cast<fxp>(out_sum));
+    });
+}
+
 rmx_status rmx_evaluate_sn_moves(rmx_graph *g, const int32_t *part, int32_t n_sn, const int32_t *sn_part,
                                  const uint8_t *allow_new, int32_t *best_mod, double *best_delta) {
     return guard([&] {

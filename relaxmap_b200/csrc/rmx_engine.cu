@@ -77,13 +77,30 @@ __global__ void k_project(int32_t n, const int32_t *node_sn, const int32_t *sn_m
 
 // Intra-module links for the coarse-tune sub-networks (generate_network_from_module,
 // OmpRelaxmap.cpp:664-684): per row, the links whose other end shares the module.
-// live (may be null): rows of instances that have stopped (inst) have none.
+// A warp per row; rows of more than kIntraLong links (R-MAT hubs) are listed in
+// chunks of that many for k_intra_long instead of keeping one warp, whose chain
+// of 32 links a step the rest of the chip waited for (row << 32 | chunk; items
+// null where the level has no hub units, so no such row). Sub-networks and
+// conversions of a run: R-MAT scale 20 14.1 -> 12.2 ms, scale 22 47.6 -> 43.2. live (may
+// be null): rows of instances that have stopped (inst) have none.
+constexpr int64_t kIntraLong = 4096;
+
+__device__ __forceinline__ bool list_long(int64_t *items, unsigned long long *n_items, int64_t u, int64_t d, int lane) {
+    if (!items || d <= kIntraLong) return false;
+    const int64_t nc = (d + kIntraLong - 1) / kIntraLong;
+    unsigned long long k0 = 0;
+    if (lane == 0) k0 = atomicAdd(n_items, (unsigned long long)nc);
+    k0 = __shfl_sync(kFull, k0, 0);
+    for (int64_t c = lane; c < nc; c += 32) items[k0 + c] = (u << 32) | c;
+    return true;
+}
+
 __global__ void k_intra_count(int32_t n, const int64_t *off, const int32_t *nbr, const int32_t *mod, int64_t *cnt,
-                              const int32_t *inst, const uint8_t *live) {
+                              const int32_t *inst, const uint8_t *live, int64_t *items, unsigned long long *n_items) {
     const int lane = threadIdx.x & 31;
     const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t u = gw; u < n; u += nw) {
-        if (live && !live[inst[u]]) {
+        if ((live && !live[inst[u]]) || list_long(items, n_items, u, off[u + 1] - off[u], lane)) {
             if (lane == 0) cnt[u] = 0;
             continue;
         }
@@ -98,7 +115,7 @@ __global__ void k_intra_count(int32_t n, const int64_t *off, const int32_t *nbr,
 
 __global__ void k_intra_fill(int32_t n, const int64_t *off, const int32_t *nbr, const fx_t *fx, const int32_t *mod,
                              const int64_t *noff, int32_t *nnbr, fx_t *nfx, fx_t *row_sum, const int32_t *inst,
-                             const uint8_t *live) {
+                             const uint8_t *live, bool long_rows) {
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
     const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -106,7 +123,8 @@ __global__ void k_intra_fill(int32_t n, const int64_t *off, const int32_t *nbr, 
         const int32_t m = mod[u];
         int64_t pos = noff[u];
         fx_t sum = 0;
-        const int64_t end = !live || live[inst[u]] ? off[u + 1] : off[u];
+        const bool none = (live && !live[inst[u]]) || (long_rows && off[u + 1] - off[u] > kIntraLong);
+        const int64_t end = none ? off[u] : off[u + 1];
         for (int64_t base = off[u]; base < end; base += 32) {
             const int64_t e = base + lane;
             const bool keep = e < end && mod[nbr[e]] == m;
@@ -122,6 +140,48 @@ __global__ void k_intra_fill(int32_t n, const int64_t *off, const int32_t *nbr, 
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
         if (row_sum && lane == 0) row_sum[u] = sum;
+    }
+}
+
+// The listed chunks, a block each: counted into cnt (FILL false) or, from
+// noff[row] + fill[row] on, written (rows are in no particular order).
+template <bool FILL>
+__global__ void __launch_bounds__(256) k_intra_long(const int64_t *items, const unsigned long long *n_items,
+                                                    const int64_t *off, const int32_t *nbr, const fx_t *fx,
+                                                    const int32_t *mod, unsigned long long *cnt, const int64_t *noff,
+                                                    unsigned *fill, int32_t *nnbr, fx_t *nfx, fx_t *row_sum) {
+    const int lane = threadIdx.x & 31;
+    const int64_t n = (int64_t)*n_items;
+    for (int64_t k = blockIdx.x; k < n; k += gridDim.x) {
+        const int64_t u = items[k] >> 32, e0 = off[u] + (items[k] & 0xffffffffll) * kIntraLong,
+                      e1 = min(off[u + 1], e0 + kIntraLong);
+        const int32_t m = mod[u];
+        unsigned c = 0;
+        fx_t sum = 0;
+        for (int64_t b = e0 + (threadIdx.x & ~31); b < e1; b += 256) {  // warp-uniform
+            const int64_t e = b + lane;
+            const int32_t v = e < e1 ? nbr[e] : 0;
+            const bool keep = e < e1 && mod[v] == m;
+            const unsigned bal = __ballot_sync(kFull, keep);
+            c += __popc(bal);
+            if (FILL && bal) {
+                unsigned base = 0;
+                if (lane == 0) base = atomicAdd(fill + u, (unsigned)__popc(bal));
+                base = __shfl_sync(kFull, base, 0);
+                if (keep) {
+                    const int64_t q = noff[u] + base + __popc(bal & ((1u << lane) - 1u));
+                    nnbr[q] = v;
+                    nfx[q] = fx[e];
+                    sum += fx[e];
+                }
+            }
+        }
+        if (!FILL && lane == 0 && c) atomicAdd(cnt + u, (unsigned long long)c);
+        if (FILL && row_sum) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
+            if (lane == 0 && sum) atomic_add_fx(row_sum + u, sum);
+        }
     }
 }
 
@@ -1272,32 +1332,9 @@ bool rmx_graph::convert_level(Level &from, int64_t from_hubs, const int32_t *row
 // starting in their parent module.
 void rmx_graph::generate_sub_modules() {
     const NvtxRange range("rmx coarse-tune");
-    timers.begin(kTimerCoarsen, stream);
-    count_units(node_lv, mods, stream);  // nodes per parent module
-    size_t mk = scratch.mark();
-    int64_t *cnt_out = scratch.alloc<int64_t>(N + 1), *cnt_in = scratch.alloc<int64_t>(N + 1);
-    const unsigned GW = blocks_for((int64_t)N * 32, 256, num_sms() * 32);
-    RMX_CUDA(cudaMemsetAsync(cnt_out + N, 0, sizeof(int64_t), stream));
-    RMX_CUDA(cudaMemsetAsync(cnt_in + N, 0, sizeof(int64_t), stream));
     const uint8_t *const lv = K > 1 ? inst1.active : nullptr;  // the instances of the next superstep
-    k_intra_count<<<GW, 256, 0, stream>>>(N, out_off, out_dst, nmod, cnt_out, node_inst, lv);
-    RMX_LAUNCHED();
-    k_intra_count<<<GW, 256, 0, stream>>>(N, in_off, in_src, nmod, cnt_in, node_inst, lv);
-    RMX_LAUNCHED();
-    scan_exclusive(cnt_out, sub_lv.out_off, N + 1, nullptr, scratch, stream);
-    scan_exclusive(cnt_in, sub_lv.in_off, N + 1, nullptr, scratch, stream);
-    fx_t *intra_out = reinterpret_cast<fx_t *>(cnt_out);  // counts are consumed by the scans above
-    k_intra_fill<<<GW, 256, 0, stream>>>(N, out_off, out_dst, out_fx, nmod, sub_lv.out_off, sub_lv.out_dst,
-                                         sub_lv.out_fx, intra_out, node_inst, lv);
-    RMX_LAUNCHED();
-    k_intra_fill<<<GW, 256, 0, stream>>>(N, in_off, in_src, in_fx, nmod, sub_lv.in_off, sub_lv.in_src, sub_lv.in_fx,
-                                         nullptr, node_inst, lv);
-    RMX_LAUNCHED();
-    k_sub_attr<<<blocks_for(N, 256, num_sms() * 32), 256, 0, stream>>>(N, nattr, intra_out, sub_lv.attr);
-    RMX_LAUNCHED();
-    scratch.release(mk);
-    sub_lv.n = N;
-    RMX_CUDA(cudaMemcpyAsync(&sub_lv.m, sub_lv.out_off + N, sizeof(int64_t), cudaMemcpyDeviceToHost, stream));
+    timers.begin(kTimerCoarsen, stream);
+    build_sub_level();
     // sub-problem state: singleton sub-modules, per-parent code lengths
     init_singletons(sub_lv, submods, stream);
     RMX_CUDA(cudaMemsetAsync(instsub.s0, 0, sizeof(fx_t) * N, stream));
@@ -1353,7 +1390,7 @@ void rmx_graph::generate_sub_modules() {
         return;
     }
     count_units(sub_lv, submods, stream);
-    mk = scratch.mark();
+    const size_t mk = scratch.mark();
     int64_t *snid = scratch.alloc<int64_t>(N + 1);
     k_flags_nonempty<<<blocks_for(N, 256, num_sms() * 32), 256, 0, stream>>>(N, submods.count, snid);
     RMX_LAUNCHED();
@@ -1386,6 +1423,64 @@ void rmx_graph::generate_sub_modules() {
     }
     scratch.release(mk);
     timers.end(kTimerCoarsen, stream);
+}
+
+// The level of the sub-networks: every node's links to nodes of its own module.
+void rmx_graph::build_sub_level() {
+    count_units(node_lv, mods, stream);  // nodes per parent module
+    const size_t mk = scratch.mark();
+    int64_t *cnt_out = scratch.alloc<int64_t>(N + 1), *cnt_in = scratch.alloc<int64_t>(N + 1);
+    const unsigned GW = blocks_for((int64_t)N * 32, 256, num_sms() * 32);
+    RMX_CUDA(cudaMemsetAsync(cnt_out + N, 0, sizeof(int64_t), stream));
+    RMX_CUDA(cudaMemsetAsync(cnt_in + N, 0, sizeof(int64_t), stream));
+    const uint8_t *const lv = K > 1 ? inst1.active : nullptr;  // the instances of the next superstep
+    const bool long_rows = node_hubs > 0;
+    int64_t *items[2] = {nullptr, nullptr};  // chunks of long rows, of the out-links then of the in-links
+    unsigned long long *n_items = nullptr;
+    if (long_rows) {
+        n_items = scratch.alloc<unsigned long long>(2);
+        RMX_CUDA(cudaMemsetAsync(n_items, 0, 2 * sizeof(unsigned long long), stream));
+        for (int64_t *&it : items) it = scratch.alloc<int64_t>(2 * (size_t)(E / kIntraLong) + 2);
+    }
+    const unsigned GL = num_sms() * 8;
+    k_intra_count<<<GW, 256, 0, stream>>>(N, out_off, out_dst, nmod, cnt_out, node_inst, lv, items[0], n_items);
+    RMX_LAUNCHED();
+    k_intra_count<<<GW, 256, 0, stream>>>(N, in_off, in_src, nmod, cnt_in, node_inst, lv, items[1], n_items + 1);
+    RMX_LAUNCHED();
+    if (long_rows) {
+        k_intra_long<false><<<GL, 256, 0, stream>>>(items[0], n_items, out_off, out_dst, nullptr, nmod,
+                                                    reinterpret_cast<unsigned long long *>(cnt_out), nullptr, nullptr,
+                                                    nullptr, nullptr, nullptr);
+        RMX_LAUNCHED();
+        k_intra_long<false><<<GL, 256, 0, stream>>>(items[1], n_items + 1, in_off, in_src, nullptr, nmod,
+                                                    reinterpret_cast<unsigned long long *>(cnt_in), nullptr, nullptr,
+                                                    nullptr, nullptr, nullptr);
+        RMX_LAUNCHED();
+    }
+    scan_exclusive(cnt_out, sub_lv.out_off, N + 1, nullptr, scratch, stream);
+    scan_exclusive(cnt_in, sub_lv.in_off, N + 1, nullptr, scratch, stream);
+    fx_t *intra_out = reinterpret_cast<fx_t *>(cnt_out);  // counts are consumed by the scans above
+    unsigned *const fill_out = reinterpret_cast<unsigned *>(cnt_in), *const fill_in = fill_out + N;  // how far each long row is filled
+    if (long_rows) RMX_CUDA(cudaMemsetAsync(fill_out, 0, 2 * sizeof(unsigned) * (size_t)N, stream));
+    k_intra_fill<<<GW, 256, 0, stream>>>(N, out_off, out_dst, out_fx, nmod, sub_lv.out_off, sub_lv.out_dst,
+                                         sub_lv.out_fx, intra_out, node_inst, lv, long_rows);
+    RMX_LAUNCHED();
+    k_intra_fill<<<GW, 256, 0, stream>>>(N, in_off, in_src, in_fx, nmod, sub_lv.in_off, sub_lv.in_src, sub_lv.in_fx,
+                                         nullptr, node_inst, lv, long_rows);
+    RMX_LAUNCHED();
+    if (long_rows) {
+        k_intra_long<true><<<GL, 256, 0, stream>>>(items[0], n_items, out_off, out_dst, out_fx, nmod, nullptr,
+                                                   sub_lv.out_off, fill_out, sub_lv.out_dst, sub_lv.out_fx, intra_out);
+        RMX_LAUNCHED();
+        k_intra_long<true><<<GL, 256, 0, stream>>>(items[1], n_items + 1, in_off, in_src, in_fx, nmod, nullptr,
+                                                   sub_lv.in_off, fill_in, sub_lv.in_src, sub_lv.in_fx, nullptr);
+        RMX_LAUNCHED();
+    }
+    k_sub_attr<<<blocks_for(N, 256, num_sms() * 32), 256, 0, stream>>>(N, nattr, intra_out, sub_lv.attr);
+    RMX_LAUNCHED();
+    scratch.release(mk);
+    sub_lv.n = N;
+    RMX_CUDA(cudaMemcpyAsync(&sub_lv.m, sub_lv.out_off + N, sizeof(int64_t), cudaMemcpyDeviceToHost, stream));
 }
 
 // One superstep (stochastic_greedy_partition, OmpRelaxmap.cpp:263-429).
@@ -1673,6 +1768,32 @@ void rmx_graph::coarsen_engine_hook(const int32_t *part_host, const int32_t *par
     }
     if (n_sn) *n_sn = ns;
     if (n_links) *n_links = m;
+}
+
+void rmx_graph::sub_level_hook(const int32_t *part_host, int64_t *n_links, int64_t *o_off, int32_t *o_dst, fx_t *o_fx,
+                               int64_t *i_off, int32_t *i_src, fx_t *i_fx, fx_t *out_sum) {
+    initiate();
+    check_partition(part_host);
+    RMX_CUDA(cudaMemcpyAsync(nmod, part_host, sizeof(int32_t) * N, cudaMemcpyHostToDevice, stream));
+    module_stats_from_units(node_lv, mods, stream);
+    RMX_CUDA(cudaMemsetAsync(inst1.active, 1, (size_t)K, stream));
+    ensure_hub_table(node_lv);  // the bin bounds may have changed since initiate
+    build_sub_level();
+    RMX_CUDA(cudaStreamSynchronize(stream));
+    const size_t m = (size_t)sub_lv.m, no = sizeof(int64_t) * ((size_t)N + 1);
+    std::vector<Stat4> st(N);
+    RMX_CUDA(cudaMemcpyAsync(st.data(), sub_lv.attr, sizeof(Stat4) * N, cudaMemcpyDeviceToHost, stream));
+    RMX_CUDA(cudaMemcpyAsync(o_off, sub_lv.out_off, no, cudaMemcpyDeviceToHost, stream));
+    RMX_CUDA(cudaMemcpyAsync(i_off, sub_lv.in_off, no, cudaMemcpyDeviceToHost, stream));
+    if (m > 0) {
+        RMX_CUDA(cudaMemcpyAsync(o_dst, sub_lv.out_dst, sizeof(int32_t) * m, cudaMemcpyDeviceToHost, stream));
+        RMX_CUDA(cudaMemcpyAsync(o_fx, sub_lv.out_fx, sizeof(fx_t) * m, cudaMemcpyDeviceToHost, stream));
+        RMX_CUDA(cudaMemcpyAsync(i_src, sub_lv.in_src, sizeof(int32_t) * m, cudaMemcpyDeviceToHost, stream));
+        RMX_CUDA(cudaMemcpyAsync(i_fx, sub_lv.in_fx, sizeof(fx_t) * m, cudaMemcpyDeviceToHost, stream));
+    }
+    RMX_CUDA(cudaStreamSynchronize(stream));
+    for (int32_t u = 0; u < N; u++) out_sum[u] = st[u].OUT;
+    *n_links = sub_lv.m;
 }
 
 void rmx_graph::evaluate_sn_hook(const int32_t *part_host, int32_t n_sn, const int32_t *sn_part_host,

@@ -177,6 +177,10 @@ struct rmx_graph {
     void coarsen_engine_hook(const int32_t *part, const int32_t *part2, int32_t *n_sn, int64_t *n_links,
                              int32_t *sn_of_mod, int64_t *o_off, int32_t *o_dst, rmx::fx_t *o_fx, int64_t *i_off,
                              int32_t *i_src, rmx::fx_t *i_fx, rmx::fx_t *sn_stat);
+    // The coarse-tune level of a given partition: links inside modules, rows
+    // unordered, and every node's sum of them.
+    void sub_level_hook(const int32_t *part, int64_t *n_links, int64_t *o_off, int32_t *o_dst, rmx::fx_t *o_fx,
+                        int64_t *i_off, int32_t *i_src, rmx::fx_t *i_fx, rmx::fx_t *out_sum);
     // Move decisions of every super-node of the level built from part, with
     // the super-nodes assigned to modules sn_part[n_sn].
     void evaluate_sn_hook(const int32_t *part, int32_t n_sn, const int32_t *sn_part, const uint8_t *allow_new,
@@ -210,6 +214,7 @@ struct rmx_graph {
     void convert_to_supernodes(bool from_sn);
     bool convert_level(rmx::Level &from, int64_t from_hubs, const int32_t *row_mod, rmx::Level &to, const int32_t *unit_mod,
                        rmx::ModState &M, bool sub);
+    void build_sub_level();
     void generate_sub_modules();
     void project_sn_to_nodes();
     int32_t count_modules();

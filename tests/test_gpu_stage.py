@@ -102,3 +102,44 @@ def test_conversion_of_a_group_of(built_lib, links):
     got = c["in_src"].astype(np.int64) * c["n_sn"] + cols
     order = np.argsort(got)
     assert np.array_equal(got[order], key) and np.array_equal(c["in_fx"][order], want)
+
+
+@pytest.mark.parametrize("links", [4095, 4096, 4097, 8192, 8193, 20000])
+def test_links_inside_modules_of_rows_of(built_lib, links):
+    """Rows of the given number of out- and of in-links (on either side of the bound and of a chunk's end), part of
+    them inside the row's module; row 0 has links of its own module only, row 1 none, row 2 about half."""
+    from relaxmap_b200 import Graph
+    n = 24001
+    rng = np.random.default_rng(links)
+    src, dst = [np.arange(3, n)], [3 + (np.arange(3, n) * 7 + 5) % (n - 3)]
+    for u in range(3):
+        for a, b in ((src, dst), (dst, src)):
+            a.append(np.full(links, u))
+            b.append(3 + rng.permutation(n - 3)[:links])
+    src, dst = np.concatenate(src), np.concatenate(dst)
+    key = np.unique((src * np.int64(n) + dst)[src != dst])
+    src, dst = key // n, key % n
+    for mine in (0, 1, 2):
+        part = np.where(rng.random(n) < 0.5, 0, 5).astype(np.int32) if mine == 2 else np.zeros(n, dtype=np.int32)
+        part[:3] = 0
+        part[1] = 9 if mine == 1 else 0
+        with Graph.from_edges(src, dst, rng.uniform(1, 3, len(src)), n=n) as g:
+            off, gdst, _, _ = g.links()
+            f = g.initiate()["f"]
+            c = g.sub_level(part)
+        fx = np.rint(f * 2.0 ** 62).astype(np.int64)
+        row = np.repeat(np.arange(n, dtype=np.int64), np.diff(off))
+        keep = part[row] == part[gdst]
+        key = row[keep] * n + gdst[keep]
+        order = np.argsort(key)
+        rows = np.repeat(np.arange(n, dtype=np.int64), np.diff(c["out_off"]))
+        got = rows * n + c["out_dst"]
+        at = np.argsort(got)
+        assert np.array_equal(got[at], key[order]) and np.array_equal(c["out_fx"][at], fx[keep][order])
+        cols = np.repeat(np.arange(n, dtype=np.int64), np.diff(c["in_off"]))
+        got = c["in_src"].astype(np.int64) * n + cols
+        at = np.argsort(got)
+        assert np.array_equal(got[at], key[order]) and np.array_equal(c["in_fx"][at], fx[keep][order])
+        want = np.zeros(n, dtype=np.int64)
+        np.add.at(want, row[keep], fx[keep])
+        assert np.array_equal(c["out_sum"], want)
