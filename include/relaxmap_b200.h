@@ -315,7 +315,7 @@ typedef struct rmx_tuning {
     int32_t eval_mid_grid;    /* mid bin (default 8) */
     int32_t eval_block_grid;  /* block bin (default 4) */
     int32_t eval_large_grid;  /* large bin (default 2) */
-    int32_t eval_warp_grid;   /* warp bin (default 4) */
+    int32_t eval_warp_grid;   /* warp bin (default 3) */
     int32_t eval_reg_grid;    /* register bins (default 8) */
     int32_t warp_max_degree;  /* default 128 */
     int32_t mid_max_degree;   /* default 512 */

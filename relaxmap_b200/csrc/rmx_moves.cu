@@ -127,7 +127,7 @@ constexpr int kBlkT = 256, kBlkMaxDeg = 1024, kBlkCap = 2048;
 #define RMX_BLK_GRID 4
 #endif
 #ifndef RMX_WARP_GRID
-#define RMX_WARP_GRID 4
+#define RMX_WARP_GRID 3
 #endif
 #ifndef RMX_REG_GRID
 #define RMX_REG_GRID 8
@@ -137,7 +137,7 @@ constexpr int kBlkT = 256, kBlkMaxDeg = 1024, kBlkCap = 2048;
 #define RMX_REG_MINB 4
 #endif
 #ifndef RMX_WARP_MINB
-#define RMX_WARP_MINB 4
+#define RMX_WARP_MINB 3
 #endif
 #ifndef RMX_DELTA_MINB
 #define RMX_DELTA_MINB 5
@@ -833,7 +833,7 @@ __global__ void __launch_bounds__(kHubPT, RMX_HUB_MINB) k_hub_eval(EvalArgs a, H
         const int32_t u = a.list[h0 + j];
         const int64_t b0 = p.pstart[pidx], b1 = p.pstart[pidx + 1];
         const int32_t A = a.mod[u];
-        const UnitCtx c = make_ctx<true>(a.attr[u], a.mrec[A], a.inst_sum_exit[a.uinst[u]], A, p.own[j]);
+        const UnitCtx c = make_ctx(a.attr[u], a.mrec[A], a.inst_sum_exit[a.uinst[u]], A, p.own[j]);
         double best = 0.0;
         int32_t bm = INT_MAX;
         for (uint32_t R = 1;; R <<= 1) {  // R rounds; more only when a round overfills the table
@@ -952,8 +952,7 @@ __global__ void k_hub_finish(EvalArgs a, HubPlan p) {
         }
         if (lane == 0) {
             const int32_t A = a.mod[u];
-            const UnitCtx c = make_ctx<true>(a.attr[u], a.mrec[A], a.inst_sum_exit[a.uinst[u]], A,
-                                       p.own[j]);
+            const UnitCtx c = make_ctx(a.attr[u], a.mrec[A], a.inst_sum_exit[a.uinst[u]], A, p.own[j]);
             p.act[j] = (uint8_t)finish_unit(a, u, c, plogp(c.eu), plogp(c.eu + c.pu), best, bm, true);
             seen += unit_links(a, u);
             units++;

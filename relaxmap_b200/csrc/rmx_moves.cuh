@@ -82,20 +82,13 @@ __device__ __forceinline__ double candidate_delta(const UnitCtx &c, const ModRec
     return candidate_delta(c, r, sfx, [](double x, double y) { return make_double2(plogp(x), plogp(y)); });
 }
 
-// The empty-module option: exit e_u, no shared flow (Module.cpp:1072-1077).
-__device__ __forceinline__ double newmod_delta(const UnitCtx &c) {
-    const double nexm = c.eu;
-    return plogp_total(c, nexm) + c.K - 2.0 * plogp(nexm) + plogp(nexm + c.pu);
-}
-
 // alpha p + beta d.
 __device__ __forceinline__ double mix_flows(double p, double d) {
     return __fma_rn(kAlpha, p, __dmul_rn(kBeta, d));
 }
 
-// HUB: the hub pipeline's order of rounding the flow between the unit and its
-// old module (the last bit may differ from the other bins').
-template <bool HUB = false>
+// The hub pipeline's terms of a unit; its order of rounding the flow between the
+// unit and its old module differs from the other bins' in the last bit.
 __device__ __forceinline__ UnitCtx make_ctx(const Stat4 &ua, const ModRec &mA, double sum_exit, int32_t A,
                                             fx_t sA) {
     const double2 tA = mA.t;
@@ -109,8 +102,7 @@ __device__ __forceinline__ UnitCtx make_ctx(const Stat4 &ua, const ModRec &mA, d
     c.eA = mA.em;
     // outFlow + inFlow to the old module (Module.cpp:1047, :1048), sA = their link flows' sum
     const double fA = from_fx(sA), dT = TWA - c.tu;
-    const double o = HUB ? __fma_rn(kBeta, fA, __dmul_rn(c.cu, dT)) : __fma_rn(c.cu, dT, __dmul_rn(kBeta, fA));
-    const double outA_inA = __fma_rn(mix_flows(PA - c.pu, DA - du), c.tu, o);
+    const double outA_inA = __fma_rn(mix_flows(PA - c.pu, DA - du), c.tu, __fma_rn(kBeta, fA, __dmul_rn(c.cu, dT)));
     c.nexA = c.eA - c.eu + outA_inA;  // :1084
     c.sum_exit = sum_exit;
     c.K = -plogp(sum_exit) - 2.0 * (plogp(c.nexA) - tA.x) + (plogp(c.nexA + (PA - c.pu)) - tA.y);
@@ -148,10 +140,10 @@ __device__ __forceinline__ Stat4 load_stat(const Stat4 *p) {
     return r;
 }
 
-// make_ctx for a group of W >= 8 lanes (gl = lane in the group): the six
-// logarithms of a unit (old module before and after, total exit, and the two of
-// the empty-module option) are taken by six lanes in one call instead of one
-// after another by all of them. newm: newmod_delta's unit terms.
+// A unit's terms by a group of W >= 8 lanes (gl = lane in the group): its six
+// logarithms (old module before and after, total exit, and the two of the
+// empty-module option, Module.cpp:1072-1077: exit e_u, no shared flow) are taken
+// by six lanes in one call instead of one after another by all of them.
 __device__ __forceinline__ UnitCtx make_ctx_lanes(int W, const Stat4 &ua, const ModRec &mA, double DA, double sum_exit, int32_t A,
                                                   fx_t sA, int gl, double &new_exit, double &new_stay) {
     const double2 tA = mA.t;

@@ -88,7 +88,7 @@ struct StageDev {
     ModRec *rec;
     int32_t *mcount, *minst;
     int32_t K;
-    double *sum_exit, *L, *L_prev;
+    double *sum_exit, *L;
     const fx_t *s0;
     fx_t *acc;
     uint8_t *active;
@@ -964,7 +964,6 @@ void fused_stage(const Level &lv, ModState &M, InstState &I, SweepWork &W, const
     a.K = I.n;
     a.sum_exit = I.sum_exit;
     a.L = I.L;
-    a.L_prev = I.L_prev;
     a.s0 = I.s0;
     a.acc = I.acc;
     a.active = I.active;
