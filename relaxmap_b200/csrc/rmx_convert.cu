@@ -13,7 +13,10 @@
 //   destination in a shared-memory table; CSR and CSC offsets; CSR rows and,
 //   column by column, CSC entries.
 // Bound by the barriers (11 of 1.25 us) and each step's chain of dependent
-// accesses: 0.22 -> 0.075 ms on the 1000-node planted graph.
+// accesses: 0.22 -> 0.075 ms on the 1000-node planted graph. On levels of
+// millions of links by the atomics: of 0.5 ms for 7.6M links, gathering takes
+// 0.11, the sums 0.13 to 0.2 and the rows and columns 0.1 (0.3 and 0.3 where the
+// groups are 290,000 sub-modules).
 // Link sums are exact integers, rows and columns come in no particular order.
 // A group whose links do not fit the tables is left to the other path: the
 // kernel reports it and nothing it wrote is kept.
@@ -34,6 +37,10 @@ constexpr unsigned kFull = 0xffffffffu;
 constexpr int kCvT = 512, kCvWarps = kCvT / 32, kCvTab = 8192, kCvWarpTab = kCvTab / kCvWarps;
 constexpr int kCvList = 256;             // slots a warp can have filled
 constexpr int kCvIlp = 4;
+// Blocks per SM. With one, larger levels wait on the sums' shared-memory and
+// column atomics: all conversions of a run on 250,001 nodes 15.3 ms, with two
+// (64 registers, no spills) 14.9; on 400,001 nodes 39.1 and 37.9.
+constexpr int kCvBlocks = 2;
 // links of a group summed by a warp, four warps, a block in one pass, a block in several
 constexpr int kCvWarpMax = 256, kCvTeamMax = 1024, kCvBlockMax = 4096, kCvMost = 16384;
 constexpr size_t kCvSmem = (size_t)kCvTab * 12 + (size_t)kCvWarps * kCvList * sizeof(uint16_t);
@@ -60,8 +67,8 @@ struct ConvDev {
     fx_t *out_fx, *in_fx;
     // scratch
     int32_t *snid, *group;
-    unsigned *gcap, *gloff, *gcross, *rowlen, *colcnt, *colfill;
-    int32_t *sk, *rk;             // gathered links and summed rows: destination group
+    unsigned *gcap, *gloff, *gcross, *rowlen, *colcnt;
+    int32_t *sk, *rk;             // gathered links and summed rows: destination group (sk then: place in its column)
     fx_t *sq, *rq;                //   and flow
     int32_t *list;                // 3 x N: groups by the size of their team
     int64_t *blk;                 // 2 per block
@@ -141,7 +148,9 @@ __device__ __forceinline__ long long cv_before(const int64_t *blk, int k, ConvSh
 }
 
 // Sums the gathered links of group g by destination (a team of NW warps, table
-// slice from slot tab on) into a row at the start of its room in rk / rq.
+// slice from slot tab on) into a row at the start of its room in rk / rq; every
+// entry's place in its column replaces the links in sk, so that writing the
+// columns takes no second atomic.
 // Keys are taken in rounds of a power of two parts of their hash so that a
 // round's distinct keys fit; false if a list overflows all the same.
 __device__ __forceinline__ bool sum_group(const ConvDev &a, int NW, int32_t g, int tab, ConvShared &sh) {
@@ -209,7 +218,7 @@ __device__ __forceinline__ bool sum_group(const ConvDev &a, int NW, int32_t g, i
             cv_hi(s) = 0;
             a.rk[b0 + pos + q] = k;
             a.rq[b0 + pos + q] = v;
-            atomicAdd(a.colcnt + k, 1u);
+            if (R == 1) a.sk[b0 + pos + q] = (int32_t)atomicAdd(a.colcnt + k, 1u);  // every gathered link has been read
             total += v;
         }
         cv_sync(NW, bar);
@@ -219,12 +228,15 @@ __device__ __forceinline__ bool sum_group(const ConvDev &a, int NW, int32_t g, i
         for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(kFull, total, o);
         if (lane == 0 && total) atomic_add_fx(&a.attr[g].OUT, total);
     }
-    if (rank == 0) a.rowlen[g] = sh.rowpos[w0];
+    const unsigned row = sh.rowpos[w0];
+    if (rank == 0) a.rowlen[g] = row;
+    if (R > 1)  // rk is the team's own writing, ordered by cv_sync
+        for (unsigned j = rank; j < row; j += NT) a.sk[b0 + j] = (int32_t)atomicAdd(a.colcnt + a.rk[b0 + j], 1u);
     cv_sync(NW, bar);
     return ok;
 }
 
-__global__ void __launch_bounds__(kCvT, 1) k_convert(const __grid_constant__ ConvDev a) {
+__global__ void __launch_bounds__(kCvT, kCvBlocks) k_convert(const __grid_constant__ ConvDev a) {
     cg::grid_group grid = cg::this_grid();
     __shared__ ConvShared sh;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nb = (int)gridDim.x, bx = (int)blockIdx.x;
@@ -237,7 +249,7 @@ __global__ void __launch_bounds__(kCvT, 1) k_convert(const __grid_constant__ Con
     }
     for (int64_t i = gtid; i < a.N; i += gthreads) {
         a.count[i] = 0;
-        a.gcap[i] = a.gcross[i] = a.rowlen[i] = a.colcnt[i] = a.colfill[i] = 0;
+        a.gcap[i] = a.gcross[i] = a.rowlen[i] = a.colcnt[i] = 0;
     }
     grid.sync();
     for (int64_t v = gtid; v < a.N; v += gthreads) atomicAdd(a.count + a.unit_mod[v], 1);
@@ -459,7 +471,7 @@ __global__ void __launch_bounds__(kCvT, 1) k_convert(const __grid_constant__ Con
     // rows, eight lanes each (the whole warp for rows of more than 64 entries), and their entries in the columns
     auto put = [&](int32_t g, unsigned from, int64_t to, unsigned len, int r, int width) {
         for (unsigned j0 = 0; j0 < len; j0 += kCvIlp * width) {
-            int32_t b[kCvIlp];
+            int32_t b[kCvIlp], at[kCvIlp];
             fx_t q[kCvIlp];
             int64_t p[kCvIlp];
 #pragma unroll
@@ -468,12 +480,13 @@ __global__ void __launch_bounds__(kCvT, 1) k_convert(const __grid_constant__ Con
                 b[k] = -1;
                 if (j < len) {
                     b[k] = a.rk[from + j];
+                    at[k] = a.sk[from + j];
                     q[k] = a.rq[from + j];
                 }
             }
 #pragma unroll
             for (int k = 0; k < kCvIlp; k++)
-                if (b[k] >= 0) p[k] = a.in_off[b[k]] + atomicAdd(a.colfill + b[k], 1u);
+                if (b[k] >= 0) p[k] = a.in_off[b[k]] + at[k];
 #pragma unroll
             for (int k = 0; k < kCvIlp; k++)
                 if (b[k] >= 0) {
@@ -519,9 +532,9 @@ bool convert_fused(const ConvertArgs &c, ConvertResult &out, Arena &ar, cudaStre
     const size_t mk = ar.mark();
     const int32_t N = c.N;
     const int64_t m = std::max<int64_t>(c.m, 1);
-    if (ar.cap - ar.mark() < (size_t)m * 24 + (size_t)N * 40 + (size_t)c.src->n * 4 + (1 << 16))
+    if (ar.cap - ar.mark() < (size_t)m * 24 + (size_t)N * 36 + (size_t)c.src->n * 4 + (1 << 16))
         return false;  // far more nodes than links: the other path needs less scratch
-    const int nb = (int)std::max<int64_t>(1, std::min<int64_t>(num_sms(), std::max<int64_t>(m / 2048, N / 512)));
+    const int nb = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)std::min(resident[dev], kCvBlocks) * num_sms(), std::max<int64_t>(m / 2048, N / 512)));
     ConvDev a;
     a.N = N;
     a.unit_mod = c.unit_mod;
@@ -557,7 +570,6 @@ bool convert_fused(const ConvertArgs &c, ConvertResult &out, Arena &ar, cudaStre
     a.gcross = ar.alloc<unsigned>(N);
     a.rowlen = ar.alloc<unsigned>(N);
     a.colcnt = ar.alloc<unsigned>(N);
-    a.colfill = ar.alloc<unsigned>(N);
     a.sk = ar.alloc<int32_t>(m);
     a.sq = ar.alloc<fx_t>(m);
     a.rk = ar.alloc<int32_t>(m);
