@@ -709,10 +709,13 @@ static int power_blocks(int32_t n, int vec, int max_nb) {
     return (int)std::min<int64_t>(max_nb, std::max<int64_t>(1, ((int64_t)n * vec + kPowT - 1) / kPowT));
 }
 
-// Blocks of k_power launched for nb virtual blocks: all of them on large
-// graphs (six per SM: the pull wants every warp it can have); below 2^17 rows
-// half as many, each taking two (the barriers and the partial sums' readers
-// cost less: 30,001 nodes 828 -> 739 us for 50 iterations).
+// Blocks of k_power launched for nb virtual blocks: all of them (six per SM: the
+// pull wants every warp it can have), or half as many, each taking two, where a
+// virtual block has one to two and a quarter steps of rows: the barriers and the
+// partial sums' readers then cost more than the pull gains (50 iterations, half
+// and all: 60,003 nodes of degree 16 913 and 1050 us, 120,007 nodes 1217 and
+// 1309; below, 30,001 nodes 642 and 575; above, 120,007 nodes of degree 24 at 8
+// lanes a row 1746 and 1486, 180,001 nodes of degree 10 2764 and 2511 us for 102).
 template <int VEC>
 static int power_launch_grid(int32_t n, int nb) {
     static std::mutex mu;
@@ -728,7 +731,9 @@ static int power_launch_grid(int32_t n, int nb) {
         RMX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident[dev], k_power<VEC>, kPowT, 0));
     }
     if (resident[dev] < 1) throw CudaError(cudaErrorLaunchOutOfResources, "power iteration does not fit an SM");
-    const int res = std::min(resident[dev], n < (1 << 17) ? kPowGrid / 2 : kPowGrid) * num_sms();
+    const int64_t lanes = (int64_t)n * VEC, threads = (int64_t)kPowGrid * num_sms() * kPowT;
+    const bool half = lanes >= threads && 4 * lanes <= 9 * threads;
+    const int res = std::min(resident[dev], half ? kPowGrid / 2 : kPowGrid) * num_sms();
     const int turns = (nb + res - 1) / res;
     return (nb + turns - 1) / turns;
 }
