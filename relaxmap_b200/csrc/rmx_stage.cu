@@ -28,8 +28,9 @@
 // two blocks at 64 registers spilt the chain's values to local memory and took
 // 431 against 379 us per sub-batch of the 1M-node planted graph's node level,
 // and 10.8 against 6.5 us on a 44-unit level. Measured as whole runs against
-// the kernel pipeline: 1000 nodes 2.78 -> 1.97 ms, 20,011 nodes in normal mode
-// 19.0 -> 13.0 ms, 150,001 nodes 83 -> 64 ms, 1M nodes 330 -> 319 ms.
+// the kernel pipeline as it was then: 1000 nodes 2.78 -> 1.97 ms, 20,011 nodes in
+// normal mode 19.0 -> 13.0 ms, 150,001 nodes 83 -> 64 ms. Levels of more than
+// 2^23 links are left to that pipeline's kernels of 32 warps per SM.
 #include <cooperative_groups.h>
 
 #include <algorithm>
