@@ -72,8 +72,10 @@ struct ConvDev {
     fx_t *sq, *rq;                //   and flow
     int32_t *list;                // 3 x N: groups by the size of their team
     int64_t *blk;                 // 2 per block
-    // [0] super-nodes [1] links [2] not done [3..6] hub units, partitions, links, chunks
+    // [0] super-nodes [1] links [2] a group has too many links [3..6] hub units, partitions, links, chunks
     // [8..10] groups per list [11] gathered links allotted [12] groups of the block list taken
+    // [13] a list of filled slots overflowed. A word that the blocks test after a barrier is not written again before
+    // the next one: a block still on its way to the test would leave alone, and the others wait for it.
     unsigned long long *ctl;
     int64_t hub_bound, hub_part, hub_chunk, hub_max_parts;
 };
@@ -419,10 +421,10 @@ __global__ void __launch_bounds__(kCvT, kCvBlocks) k_convert(const __grid_consta
             }
             ok &= sum_group(a, NW, g, (w & ~(NW - 1)) * kCvWarpTab, sh);
         }
-        if (!ok) a.ctl[2] = 1;
+        if (!ok) a.ctl[13] = 1;
     }
     grid.sync();
-    if (__ldcg(a.ctl + 2)) return;
+    if (__ldcg(a.ctl + 13)) return;  // the same in every block
     // CSR and CSC offsets; what the level's hub units need
     const int64_t gchunk = (((int64_t)ng + nb - 1) / nb + kCvT - 1) / kCvT * kCvT;
     const int64_t g0 = min((int64_t)ng, bx * gchunk), g1 = min((int64_t)ng, g0 + gchunk);
@@ -586,11 +588,11 @@ bool convert_fused(const ConvertArgs &c, ConvertResult &out, Arena &ar, cudaStre
     void *args[] = {(void *)&a};
     RMX_CUDA(cudaLaunchCooperativeKernel((void *)k_convert, dim3(nb), dim3(kCvT), args, kCvSmem, s));
     RMX_LAUNCHED();
-    unsigned long long r[7];
+    unsigned long long r[14];
     RMX_CUDA(cudaMemcpyAsync(r, a.ctl, sizeof r, cudaMemcpyDeviceToHost, s));
     RMX_CUDA(cudaStreamSynchronize(s));
     ar.release(mk);
-    if (r[2]) return false;
+    if (r[2] || r[13]) return false;
     out.n = (int32_t)r[0];
     out.m = (int64_t)r[1];
     for (int k = 0; k < 4; k++) out.hub[k] = (int64_t)r[3 + k];
