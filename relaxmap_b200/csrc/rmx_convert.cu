@@ -206,12 +206,17 @@ __device__ __forceinline__ bool sum_group(const ConvDev &a, int NW, int32_t g, i
                 cnt += __popc(bal);
             }
         }
-        if (cnt > kCvList) ok = false;  // only possible in rounds; the table is dropped with the launch
+        // Only possible in rounds: the entries past the list, and the table with them, are dropped with the launch.
+        // What is counted into the row is what is written to it, since the row is read back below.
+        if (cnt > kCvList) {
+            ok = false;
+            cnt = kCvList;
+        }
         cv_sync(NW, bar);
         unsigned pos = 0;
         if (lane == 0) pos = atomicAdd(&sh.rowpos[w0], (unsigned)cnt);
         pos = __shfl_sync(kFull, pos, 0);
-        for (int q = lane; q < min(cnt, kCvList); q += 32) {
+        for (int q = lane; q < cnt; q += 32) {
             const int s = tab + cv_list(q);
             const int32_t k = cv_key(s);
             const fx_t v = (fx_t)(((unsigned long long)cv_hi(s) << 32) | cv_lo(s));

@@ -143,3 +143,49 @@ def test_links_inside_modules_of_rows_of(built_lib, links):
         want = np.zeros(n, dtype=np.int64)
         np.add.at(want, row[keep], fx[keep])
         assert np.array_equal(c["out_sum"], want)
+
+
+def _mix32(x):
+    x = x.astype(np.uint32)
+    for shift, mul in ((16, 0x7feb352d), (15, 0x846ca68b)):
+        x ^= x >> np.uint32(shift)
+        x *= np.uint32(mul)
+    return x ^ (x >> np.uint32(16))
+
+
+@pytest.mark.parametrize("modules,links", [(1, 4500), (1, 16000), (40, 5000)])
+def test_conversion_of_groups_whose_ids_share_a_hash(built_lib, modules, links):
+    """Modules whose links lead to super-nodes that one of the conversion's rounds (4 up to 8192 links, 8 above)
+    takes all of: more of them per warp than its list holds, so the launch is dropped and the separate kernels
+    give the sums. With as many links to any ids the one launch is kept."""
+    from relaxmap_b200 import Graph
+    n, size, rounds = 1 << 18, 16, 4 if links <= 8192 else 8
+    members = modules * size
+    assert links / 16 > 256  # distinct ids over the 16 warps of a block, in one round
+    rng = np.random.default_rng(links)
+    part = np.arange(n, dtype=np.int32)
+    part[:members] -= part[:members] % size
+    group = np.searchsorted(np.unique(part), part)
+    ids = np.arange(members, n)
+    same = ids[(_mix32(group[ids] ^ 0x5bd1e995) >> np.uint32(7)) % rounds == 1]
+    launches = {}
+    for name, pool in (("same", same), ("any", ids)):
+        to = np.concatenate([rng.permutation(pool)[:links] for _ in range(modules)])
+        src = np.concatenate([m * size + np.arange(links) % size for m in range(modules)])
+        with Graph.from_edges(src, to, rng.uniform(1, 3, len(src)), n=n) as g:
+            off, gdst, _, _ = g.links()
+            f = g.initiate()["f"]
+            before = g.profile()["kernel_launches"]
+            c = g.coarsen_engine(part)
+            launches[name] = g.profile()["kernel_launches"] - before
+        a, b = np.repeat(group, np.diff(off)), group[gdst]
+        key = a * np.int64(c["n_sn"]) + b
+        order = np.argsort(key)  # every link leads to a super-node of its own
+        want = np.rint(f * 2.0 ** 62).astype(np.int64)[order]
+        rows = np.repeat(np.arange(c["n_sn"], dtype=np.int64), np.diff(c["out_off"])) * c["n_sn"] + c["out_dst"]
+        at = np.argsort(rows)
+        assert np.array_equal(rows[at], key[order]) and np.array_equal(c["out_fx"][at], want)
+        cols = c["in_src"].astype(np.int64) * c["n_sn"] + np.repeat(np.arange(c["n_sn"]), np.diff(c["in_off"]))
+        at = np.argsort(cols)
+        assert np.array_equal(cols[at], key[order]) and np.array_equal(c["in_fx"][at], want)
+    assert launches["same"] >= launches["any"] + 10
