@@ -303,7 +303,8 @@ rmx_status rmx_adjoint_backward(rmx_graph *g, const int32_t *part, double tau, d
  * these values (every bin's kernel loops over its units by grid stride,
  * module statistics are exact integer sums, and every bin computes the same
  * change per candidate), only the time does. rmx_set_tuning takes effect at
- * the next launch; sweep pipelines captured as CUDA graphs under other values
+ * the next stage of sweeps, also of a run in progress on another thread, which
+ * reads all values at once when a stage begins; sweep pipelines captured as CUDA graphs under other values
  * are captured again. Each grid cap must lie in [1, 64], and
  * 32 <= warp_max <= 128, warp_max <= mid_max <= 512, mid_max <= block_max <=
  * 1024, block_max <= large_max <= 4096 (the bins' table limits; an equal

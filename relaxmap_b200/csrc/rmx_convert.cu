@@ -584,11 +584,10 @@ bool convert_fused(const ConvertArgs &c, ConvertResult &out, Arena &ar, cudaStre
     a.list = ar.alloc<int32_t>(3 * (size_t)N);
     a.blk = ar.alloc<int64_t>(2 * (size_t)nb);
     a.ctl = ar.alloc<unsigned long long>(16);
-    const HubNeeds h = hub_needs_rule();
-    a.hub_bound = h.bound;
-    a.hub_part = h.part;
-    a.hub_chunk = h.chunk;
-    a.hub_max_parts = h.max_parts;
+    a.hub_bound = c.hub.bound;
+    a.hub_part = c.hub.part;
+    a.hub_chunk = c.hub.chunk;
+    a.hub_max_parts = c.hub.max_parts;
     RMX_CUDA(cudaMemsetAsync(a.ctl, 0, sizeof(unsigned long long) * 16, s));
     void *args[] = {(void *)&a};
     RMX_CUDA(cudaLaunchCooperativeKernel((void *)k_convert, dim3(nb), dim3(kCvT), args, kCvSmem, s));

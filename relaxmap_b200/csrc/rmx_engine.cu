@@ -801,12 +801,13 @@ int64_t rmx_graph::max_degree(const Level &lv) {
 // never shrunk.
 void rmx_graph::ensure_hub_table(const Level &lv) {
     level_hubs = 0;
+    work.tune = eval_tuning(&work.tune_gen);
     if (lv.n <= 0) return;
     int64_t need[4];
-    if (&lv == known_lv && known_tuning == eval_tuning_generation())
+    if (&lv == known_lv && known_tuning == work.tune_gen)
         std::copy(known_hub, known_hub + 4, need);  // counted when the level was built
     else
-        hub_level_needs(lv, need, dtmp + 12, stream);
+        hub_level_needs(lv, work.tune, need, dtmp + 12, stream);
     const int64_t units = need[0], parts = need[1], links = need[2], chunks = need[3];
     level_hubs = units;
     if (&lv == &node_lv) node_hubs = units;
@@ -938,7 +939,7 @@ void rmx_graph::run_subbatches(Level &lv, int64_t n_active, ModState &M, InstSta
         return;
     }
     const SweepGraphKey key{&lv, &M, &I, sa.allow_new, mark ? 1 : 0, sa.vthresh, ns, work.hub_gen,
-                            eval_tuning_generation()};
+                            work.tune_gen};
     SweepGraph *gr = nullptr;
     for (SweepGraph &g : sweep_graphs)
         if (g.key == key) gr = &g;
@@ -1142,7 +1143,7 @@ void rmx_graph::stage_sweeps_graph(Level &lv, bool allow_new, std::vector<double
     const int ns = sub_batches_for(lv.n);
     const StageGraphKey key{&lv,          &mods, &inst1,   allow_new ? 1 : 0, prior ? 1 : 0,
                             opt.max_iter, ns,    vthresh,  opt.threshold,     work.hub_gen,
-                            eval_tuning_generation(), scratch.mark()};
+                            work.tune_gen, scratch.mark()};
     RMX_CUDA(cudaMemcpyAsync(stage_sweeping, act.data(), (size_t)K, cudaMemcpyHostToDevice, stream));
     loop_graph(key, lv.n, [&](unsigned long long cond) { stage_body(lv, allow_new, prior, vthresh, ns, cond); });
     RMX_CUDA(cudaMemcpyAsync(L.data(), inst1.L, sizeof(double) * K, cudaMemcpyDeviceToHost, stream));
@@ -1313,13 +1314,15 @@ void rmx_graph::convert_to_supernodes(bool from_sn) {
 bool rmx_graph::convert_level(Level &from, int64_t from_hubs, const int32_t *row_mod, Level &to, const int32_t *unit_mod, ModState &M,
                               bool sub) {
     if (from.m > kConvertMaxLinks || from.m <= 0 || from_hubs > 0) return false;
-    const ConvertArgs c{N, K, sub, unit_mod, &M, mods.inst, &from, from.m, row_mod, &to, node_sn};
+    int gen = 0;
+    const HubNeeds hub = hub_needs_rule(eval_tuning(&gen));
+    const ConvertArgs c{N, K, sub, unit_mod, &M, mods.inst, &from, from.m, row_mod, &to, node_sn, hub};
     ConvertResult r;
     if (!convert_fused(c, r, scratch, stream)) return false;
     to.n = r.n;
     to.m = r.m;
     known_lv = &to;
-    known_tuning = eval_tuning_generation();
+    known_tuning = gen;
     std::copy(r.hub, r.hub + 4, known_hub);
     return true;
 }
@@ -1358,7 +1361,7 @@ void rmx_graph::generate_sub_modules() {
         if (fused && opt.max_iter > 0) run_fused(sub_lv, submods, instsub, false, false, true, 0.0, nsg, nullptr);
         if (!fused && stage_graph_ok(sub_lv) && opt.max_iter > 0) {
             const StageGraphKey key{&sub_lv, &submods, &instsub, 0, 0, opt.max_iter, nsg, 0.0, opt.threshold,
-                                    work.hub_gen, eval_tuning_generation(), scratch.mark()};
+                                    work.hub_gen, work.tune_gen, scratch.mark()};
             loop_graph(key, N, [&](unsigned long long cond) { subtune_body(nsg, cond); });
         }
         for (int iter = 0; iter < opt.max_iter && !fused && !stage_graph_ok(sub_lv); iter++) {

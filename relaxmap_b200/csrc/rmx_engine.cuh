@@ -176,6 +176,20 @@ struct Timers {
 };
 
 
+// Launch shape of move evaluation, process-wide; a stage of sweeps reads it once
+// (SweepWork::tune):
+// the grid cap of each bin in blocks per SM, and the degree bounds that
+// assign units to the warp, mid, block and large bins (units above large_max
+// go to the hub bin). Results do not depend on them (each bin's kernel loops
+// over its units by grid stride, every bin computes the same exact integer
+// sums and the same change per candidate), only the time does. The hub bin's
+// grid is not tuned: its global table slices are indexed by block.
+struct EvalTuning {
+    int mid, block, large, warp, reg;              // grid caps
+    int warp_max, mid_max, block_max, large_max;   // degree bounds (at most 128, 512, 1024, 4096)
+    int hub_part;                                  // mean links per partition of a hub unit / huge group
+};
+
 // Per-level sweep workspace (sized for the largest level: N units, N modules).
 struct SweepWork {
     int32_t *list = nullptr, *list2 = nullptr;  // active units; active units grouped by bucket
@@ -211,44 +225,34 @@ struct SweepWork {
     std::vector<int64_t> bucket_host;  // host copy of bucket_off after bucket_units
     uint32_t *dparams = nullptr;       // device {stamp, hseed} per sub-batch of the current sweep
     uint32_t hparams[64] = {};         // host staging of dparams
+    // The tuning and its generation as ensure_hub_table read them for the level: the hub arrays are sized, the units
+    // assigned to bins and the kernels chosen by the same bounds, whatever another thread sets meanwhile.
+    EvalTuning tune{};
+    int tune_gen = 0;
     cudaStream_t aux[5] = {};  // concurrent degree bins
     cudaEvent_t fork = nullptr, join[5] = {};
 };
 
 void configure_eval_kernels();
-// What the hub pipeline needs for a level: hub units (above
-// block_bin_max_degree), their partitions, their links and their link chunks
+// What the hub pipeline needs for a level under tuning t: hub units (above
+// large_max), their partitions, their links and their link chunks
 // (out[0..3]); one device reduction, then a sync.
-void hub_level_needs(const Level &L, int64_t *out, int64_t *dev_tmp, cudaStream_t s);
+void hub_level_needs(const Level &L, const EvalTuning &t, int64_t *out, int64_t *dev_tmp, cudaStream_t s);
 
 // What hub_level_needs counts: units above bound, parts of part links (at most
 // max_parts), chunks of chunk links.
 struct HubNeeds {
     int64_t bound, part, chunk, max_parts;
 };
-HubNeeds hub_needs_rule();
+HubNeeds hub_needs_rule(const EvalTuning &t);
 
-// Launch shape of move evaluation, process-wide and read at every launch:
-// the grid cap of each bin in blocks per SM, and the degree bounds that
-// assign units to the warp, mid, block and large bins (units above large_max
-// go to the hub bin). Results do not depend on them (each bin's kernel loops
-// over its units by grid stride, every bin computes the same exact integer
-// sums and the same change per candidate), only the time does. The hub bin's
-// grid is not tuned: its global table slices are indexed by block.
-struct EvalTuning {
-    int mid, block, large, warp, reg;              // grid caps
-    int warp_max, mid_max, block_max, large_max;   // degree bounds (at most 128, 512, 1024, 4096)
-    int hub_part;                                  // mean links per partition of a hub unit / huge group
-};
-EvalTuning eval_tuning();
+// The current setting; gen (may be null): its generation, read together with it.
+EvalTuning eval_tuning(int *gen = nullptr);
 // Throws std::invalid_argument unless every grid cap lies in [1, 64] and
 // 32 <= warp_max <= mid_max <= block_max <= large_max, each within its bin's
 // table limit, and 64 <= hub_part <= 2^30.
+// Every call changes the generation (part of the sweep graph cache key).
 void set_eval_tuning(const EvalTuning &t);
-// Changes with every set_eval_tuning (part of the sweep graph cache key).
-int eval_tuning_generation();
-// Units above this degree need the hub bin's global tables.
-int64_t block_bin_max_degree();
 void all_units(int32_t n, SweepWork &W, cudaStream_t s);
 // host_counts: also copy the bin offsets to W.bucket_host (one stream sync).
 void bucket_units(const Level &L, SweepWork &W, int64_t n_active, uint32_t seed, int nsub, Arena &ar, cudaStream_t s,
@@ -324,6 +328,7 @@ struct ConvertArgs {
     const int32_t *row_mod;      // module of every unit of src, or null if its units are the nodes
     Level *dst;
     int32_t *node_sn;
+    HubNeeds hub;                // what ConvertResult::hub counts
 };
 struct ConvertResult {
     int32_t n = 0;

@@ -33,7 +33,7 @@ struct SweepGraphKey {
     double vthresh;
     int nsub;
     int64_t hub_gen;  // the hub arrays' allocation: graphs hold their addresses
-    int tuning_gen;  // eval_tuning_generation() at capture: grid sizes are part of the graph
+    int tuning_gen;  // the tuning's generation at capture: grid sizes are part of the graph
     bool operator==(const SweepGraphKey &o) const {
         return lv == o.lv && M == o.M && I == o.I && allow_new == o.allow_new && mark == o.mark &&
                vthresh == o.vthresh && nsub == o.nsub && hub_gen == o.hub_gen &&

@@ -1435,15 +1435,13 @@ __global__ void k_hub_level(int32_t n, const int64_t *out_off, const int64_t *in
     }
 }
 
-HubNeeds hub_needs_rule() {
-    const EvalTuning t = eval_tuning();
+HubNeeds hub_needs_rule(const EvalTuning &t) {
     return {t.large_max, t.hub_part, kHubCh, kMaxParts};
 }
 
-void hub_level_needs(const Level &L, int64_t *out, int64_t *dev_tmp, cudaStream_t s) {
+void hub_level_needs(const Level &L, const EvalTuning &t, int64_t *out, int64_t *dev_tmp, cudaStream_t s) {
     unsigned long long *acc = reinterpret_cast<unsigned long long *>(dev_tmp);
     RMX_CUDA(cudaMemsetAsync(acc, 0, 4 * sizeof(unsigned long long), s));
-    const EvalTuning t = eval_tuning();
     k_hub_level<<<blocks_for(L.n, 256, num_sms() * 8), 256, 0, s>>>(L.n, L.out_off, L.in_off, t.large_max, t.hub_part,
                                                                     acc);
     RMX_LAUNCHED();
@@ -1458,8 +1456,9 @@ int g_tuning_gen = 0;
 std::mutex g_tuning_mu;  // guards g_tuning and g_tuning_gen
 }  // namespace
 
-EvalTuning eval_tuning() {
+EvalTuning eval_tuning(int *gen) {
     std::lock_guard<std::mutex> lk(g_tuning_mu);
+    if (gen) *gen = g_tuning_gen;
     return g_tuning;
 }
 
@@ -1478,11 +1477,6 @@ void set_eval_tuning(const EvalTuning &t) {
     g_tuning_gen++;
 }
 
-int eval_tuning_generation() {
-    std::lock_guard<std::mutex> lk(g_tuning_mu);
-    return g_tuning_gen;
-}
-int64_t block_bin_max_degree() { return eval_tuning().large_max; }
 
 constexpr size_t kBlkSmem = table_bytes(kBlkCap);
 constexpr size_t kMidSmem = table_bytes(kMidCap);
@@ -1533,7 +1527,7 @@ static void launch_eval(EvalArgs a, const int64_t *bucket_off, int first_bucket,
                   n_warp = cnt(kBinWarp, kBinWarp + 1), n_reg = cnt(kBinReg8, kBinReg32 + 1);
     // streams: 0 block, 1 large, 2 warp, 3 mid, 4 hub, the caller's stream the register bins
     const bool use[5] = {n_blk > 0, n_lrg > 0, n_warp > 0, n_mid > 0, n_hub > 0};
-    const EvalTuning tg = eval_tuning();
+    const EvalTuning &tg = W.tune;
     int streams = n_reg > 0 ? 1 : 0;
     for (bool b : use) streams += b ? 1 : 0;
     const bool fork = streams > 1;
@@ -1684,7 +1678,7 @@ __global__ void k_ranges(const int64_t *bucket_off, int nsub, int64_t *ranges) {
 void bucket_units(const Level &L, SweepWork &W, int64_t n_active, uint32_t seed, int nsub, Arena &ar,
                   cudaStream_t s, bool host_counts) {
     if (nsub * kBins > 256) throw std::invalid_argument("too many sub-batches");
-    const EvalTuning t = eval_tuning();
+    const EvalTuning &t = W.tune;
     const BinBounds bb{t.warp_max, t.mid_max, t.block_max, t.large_max};
     k_bucket<<<blocks_for(n_active, 256, num_sms() * 32), 256, 0, s>>>(W.list, W.counters + kCntActive, L.out_off,
                                                                        L.in_off, seed, nullptr, nsub, bb, W.bucket);
@@ -1703,7 +1697,7 @@ void bucket_units(const Level &L, SweepWork &W, int64_t n_active, uint32_t seed,
 void bucket_units_dev(const Level &L, SweepWork &W, int64_t n_max, const uint32_t *seed_dev, int nsub, Arena &ar,
                       cudaStream_t s) {
     if (nsub * kBins > 256) throw std::invalid_argument("too many sub-batches");
-    const EvalTuning t = eval_tuning();
+    const EvalTuning &t = W.tune;
     const BinBounds bb{t.warp_max, t.mid_max, t.block_max, t.large_max};
     k_bucket<<<blocks_for(n_max, 256, num_sms() * 32), 256, 0, s>>>(W.list, W.counters + kCntActive, L.out_off,
                                                                     L.in_off, 0u, seed_dev, nsub, bb, W.bucket);
@@ -1806,7 +1800,7 @@ void sweep_subbatch(const Level &L, ModState &M, const InstState &I, SweepWork &
         RMX_CUDA(cudaStreamWaitEvent(W.aux[4], W.fork, 0));
         da.beg = bo + kBinHub;
         da.end = bo + kBins;
-        k_delta_hub<<<num_sms() * 8, 256, 0, W.aux[4]>>>(da, hub_plan(W, eval_tuning()));
+        k_delta_hub<<<num_sms() * 8, 256, 0, W.aux[4]>>>(da, hub_plan(W, W.tune));
         RMX_LAUNCHED();
         RMX_CUDA(cudaEventRecord(W.join[4], W.aux[4]));
     }

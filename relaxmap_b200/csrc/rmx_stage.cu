@@ -838,7 +838,9 @@ __global__ void __launch_bounds__(kSwT, RMX_STAGE_MINB) k_stage(const __grid_con
                 apply_light(a, sc.stamp, h ? 8 : 32, bo[h ? kBinReg8 : kBinWarp], bo[h ? kBinWarp : kBinMid],
                             w * nb + bx, nb * kSwWarps);
             grid.sync();
-            for (int64_t i = bo[0] + gtid; i < bo[kBins]; i += gthreads) {
+            // the hub bin, which the evaluation has no part for and so proposes nothing, is left out (the host
+            // takes no level with hub units here)
+            for (int64_t i = bo[0] + gtid; i < bo[kBinHub]; i += gthreads) {
                 const int32_t p = a.tgt[i];
                 if (p == -1) continue;
                 const int32_t u = a.urec[i].u, A = a.urec[i].A;
@@ -986,8 +988,7 @@ void fused_stage(const Level &lv, ModState &M, InstState &I, SweepWork &W, const
     a.run_seed = f.run_seed;
     a.stamp0 = f.stamp;
     a.sweep0 = f.sweep_no;
-    const EvalTuning tg = eval_tuning();
-    a.bb = BinBounds{tg.warp_max, tg.mid_max, tg.block_max, tg.large_max};
+    a.bb = BinBounds{W.tune.warp_max, W.tune.mid_max, W.tune.block_max, W.tune.large_max};
     a.set = ar.alloc<SweepSet>(2);
     a.ctl = ctl;
     // Enough blocks that every warp of a sub-batch's evaluation has about four units or 128

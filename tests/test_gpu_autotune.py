@@ -60,3 +60,34 @@ def test_autotune_end_to_end(graph, tmp_path):
     save(res, p)
     assert load(p) == res["tuning"]
     assert get_tuning() == res["tuning"]
+
+
+def test_bounds_changed_during_runs(graph):
+    """Another thread moves the bin bounds between "no hub units" and "every unit above 32 links is one"
+    while runs are in progress: each stage goes by the values it read when it began, so every run gives
+    the same result."""
+    import threading
+    from relaxmap_b200 import set_tuning
+    from relaxmap_b200.autotune import DEFAULTS
+    G = graph
+    set_tuning(**DEFAULTS)
+    ref = G.optimize(seed=3)
+    stop = threading.Event()
+
+    def change():
+        low = dict(warp_max_degree=32, mid_max_degree=32, block_max_degree=32, large_max_degree=32)
+        while not stop.is_set():
+            for values in (low, DEFAULTS):
+                set_tuning(**values)
+
+    t = threading.Thread(target=change)
+    t.start()
+    try:
+        for _ in range(20):
+            G.reset_flow()
+            r = G.optimize(seed=3)
+            assert r["L"] == ref["L"]
+            np.testing.assert_array_equal(r["part"], ref["part"])
+    finally:
+        stop.set()
+        t.join()
