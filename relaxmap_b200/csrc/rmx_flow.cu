@@ -265,7 +265,55 @@ __device__ __forceinline__ double warp_sum_parts(const double *parts, int nb, in
     return v;
 }
 
+// warp_sum_parts over shared memory.
+__device__ __forceinline__ double shared_sum_parts(const double *parts, int nb, int lane) {
+    double v = 0.0;
+#pragma unroll 4
+    for (int i = lane; i < nb; i += 32) v += parts[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+    return v;
+}
+
 constexpr int kPowT = 256;
+
+// out[k] = the sum of parts[k] as warp_sum_parts forms it, in every thread of the
+// block (K = 1 or 2). FEW: at most kPowFew partial sums, as many as two blocks per
+// SM; a thread loads one of each (a warp's threads two) and the warps add from
+// shared memory, one latency of L2 where a warp that loads its own 4 to 9 pays
+// two. A form of k_power of its own: two blocks per SM leave room for 128
+// registers, and a choice at run time took some from the pull of larger graphs
+// (120,000 nodes 1016 and 976 us). 50 iterations, this form and the other: 8,192
+// nodes 346 and 446 us, 12,000 nodes 364 and 479, 16,000 nodes 378 and 490,
+// 18,432 nodes 377 and 423.
+constexpr int kPowFew = kPowT + 32;
+template <bool FEW, int K>
+__device__ __forceinline__ void block_sum_parts(const double *const (&parts)[K], int nb, double *out,
+                                                double (*staged)[kPowFew]) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (FEW) {
+        const int i = threadIdx.x, i2 = i + kPowT;
+        double t[K], t2[K];
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            if (i < nb) t[k] = __ldcg(parts[k] + i);
+            if (i2 < nb) t2[k] = __ldcg(parts[k] + i2);
+        }
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            if (i < nb) staged[k][i] = t[k];
+            if (i2 < nb) staged[k][i2] = t2[k];
+        }
+        __syncthreads();
+    }
+    if (warp < K) {
+        const double *const p = warp == 0 ? parts[0] : parts[K - 1];
+        const double v = FEW ? shared_sum_parts(staged[warp], nb, lane) : warp_sum_parts(p, nb, lane);
+        if (lane == 0) out[warp] = v;
+    }
+    __syncthreads();
+}
+
 // The iteration's sums (total flow, L1 change, dangling mass) are formed per
 // "virtual" block of kPowT threads of a fixed grid, kPowGrid such blocks per
 // SM, and added in block order: their rounding, which the 1e-15 stop rule sits
@@ -301,15 +349,16 @@ struct PowGather {
     double *xc = nullptr;
 };
 
-template <int VEC>
-__global__ void __launch_bounds__(kPowT, RMX_POW_MINB) k_power(const int64_t *__restrict__ in_off, const int32_t *__restrict__ in_src,
+// FEW: at most kPowFew virtual blocks.
+template <int VEC, bool FEW>
+__global__ void __launch_bounds__(kPowT, FEW ? 2 : RMX_POW_MINB) k_power(const int64_t *__restrict__ in_off, const int32_t *__restrict__ in_src,
                                                  const double *__restrict__ in_w, const double *__restrict__ tw,
                                                  const uint8_t *__restrict__ dang, int32_t n, double *x, double *y,
                                                  double *parts, int *iters_out, double alpha, PowSplit sp,
                                                  PowGather pg, int nb) {
     cg::grid_group grid = cg::this_grid();
     __shared__ double sh[32];
-    __shared__ double shared_sum[2];
+    __shared__ double shared_sum[2], staged[FEW ? 2 : 1][kPowFew];
     double *Sp = parts, *Dp = parts + nb, *Ep = parts + 2 * nb;
     const int64_t gthreads = (int64_t)nb * kPowT, nwarps = gthreads >> 5;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane / VEC, lv = lane % VEC;
@@ -332,11 +381,7 @@ __global__ void __launch_bounds__(kPowT, RMX_POW_MINB) k_power(const int64_t *__
         if (threadIdx.x == 0) Dp[vb] = dl;
     }
     grid.sync();
-    if (warp == 0) {
-        const double v = warp_sum_parts(Dp, nb, lane);
-        if (lane == 0) shared_sum[1] = v;
-    }
-    __syncthreads();
+    block_sum_parts<FEW, 1>({Dp}, nb, shared_sum + 1, staged);
     int iter = 0;
     for (;;) {
         const double D = shared_sum[1];
@@ -400,11 +445,7 @@ __global__ void __launch_bounds__(kPowT, RMX_POW_MINB) k_power(const int64_t *__
             }
         }
         grid.sync();
-        if (warp == 0) {
-            const double v = warp_sum_parts(Sp, nb, lane);
-            if (lane == 0) shared_sum[0] = v;
-        }
-        __syncthreads();
+        block_sum_parts<FEW, 1>({Sp}, nb, shared_sum, staged);
         const double S = shared_sum[0];
         for (int vb = blockIdx.x; vb < nb; vb += gridDim.x) {
             double el = 0.0, dl = 0.0;
@@ -423,11 +464,7 @@ __global__ void __launch_bounds__(kPowT, RMX_POW_MINB) k_power(const int64_t *__
             }
         }
         grid.sync();
-        if (warp < 2) {
-            const double v = warp_sum_parts(warp ? Dp : Ep, nb, lane);
-            if (lane == 0) shared_sum[warp] = v;
-        }
-        __syncthreads();
+        block_sum_parts<FEW, 2>({Ep, Dp}, nb, shared_sum, staged);
         const double diff = shared_sum[0];
         iter++;
         if (iter >= 200 || (diff <= 1.0e-15 && iter >= 50)) break;  // Module.cpp:460
@@ -561,11 +598,16 @@ static PowGather gather_copy(int32_t n, const int64_t *in_off, const int32_t *in
 // k_power, 238 us here; 3001 nodes: 397 and 290 us. Rows of more than heavy_deg
 // links are left to k_power (*iters_out = -1, nothing computed).
 constexpr int kClT = 1024, kClGroups = kClT / kPowT, kClMaxSize = 16;
-// Largest graphs: every virtual warp has one step of rows, and a block has at
-// most 8 to 16 virtual blocks; the cluster's 16 SMs then take as long per
-// iteration as the whole grid (6003 nodes, 188 virtual blocks: 470 us here, 447
-// through k_power).
-constexpr int32_t kClMaxNodes = 8192, kClMaxBlocks = 128;
+// Largest graphs: every virtual warp has one step of rows, a block has at most 8
+// to 16 virtual blocks, and above four of them (which its four groups of threads
+// take at once) a node costs the cluster as much as 32 links, until its 16 SMs
+// take as long per iteration as the whole grid. 50 iterations here and through
+// k_power: 4000 nodes and 64,000 links (four virtual blocks a block) 337 and 375
+// us; above four, 1000 and 114,000 364 and 384, 2000 and 93,000 353 and 389, 3000
+// and 69,000 350 and 360, 4200 and 25,000 334 and 351; beyond the bound 3500 and
+// 63,000 357 and 357, 4200 and 46,000 364 and 360, 5000 and 30,000 368 and 350,
+// 6000 and 96,000 455 and 374.
+constexpr int32_t kClMaxNodes = 5200, kClMaxBlocks = 128, kClMaxCost = 5200;
 constexpr int64_t kClMaxLinks = 1 << 17;
 
 __device__ __forceinline__ uint32_t cl_addr(const void *p, unsigned rank) {  // p's copy in block `rank` of the cluster
@@ -578,16 +620,6 @@ __device__ __forceinline__ void cl_store(const void *p, unsigned rank, double v)
 }
 __device__ __forceinline__ void cl_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-// warp_sum_parts over shared memory.
-__device__ __forceinline__ double cl_sum_parts(const double *parts, int nb, int lane) {
-    double v = 0.0;
-#pragma unroll 4
-    for (int i = lane; i < nb; i += 32) v += parts[i];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-    return v;
 }
 
 template <int VEC>
@@ -647,7 +679,7 @@ __global__ void __launch_bounds__(kClT, 1) k_power_cluster(const int64_t *__rest
     __syncthreads();
     send(sh[1], owne, Dp);
     cl_sync();
-    double D = cl_sum_parts(Dp, nbe, lane);
+    double D = shared_sum_parts(Dp, nbe, lane);
     int iter = 0;
     for (;;) {
         const double coef = alpha + beta * D;
@@ -674,7 +706,7 @@ __global__ void __launch_bounds__(kClT, 1) k_power_cluster(const int64_t *__rest
         __syncthreads();
         send(sh[0], own, Sp);
         cl_sync();
-        const double S = cl_sum_parts(Sp, nb, lane);
+        const double S = shared_sum_parts(Sp, nb, lane);
         for (int k = grp; k < owne; k += kClGroups) {
             const int i = (k * (int)C + (int)rank) * kPowT + t;
             double el = 0.0, dl = 0.0;
@@ -695,8 +727,8 @@ __global__ void __launch_bounds__(kClT, 1) k_power_cluster(const int64_t *__rest
         send(sh[0], owne, Ep);
         send(sh[1], owne, Dp);
         cl_sync();
-        const double diff = cl_sum_parts(Ep, nbe, lane);
-        D = cl_sum_parts(Dp, nbe, lane);
+        const double diff = shared_sum_parts(Ep, nbe, lane);
+        D = shared_sum_parts(Dp, nbe, lane);
         iter++;
         if (iter >= 200 || (diff <= 1.0e-15 && iter >= 50)) break;
     }
@@ -716,7 +748,7 @@ static int power_blocks(int32_t n, int vec, int max_nb) {
 // and all: 60,003 nodes of degree 16 913 and 1050 us, 120,007 nodes 1217 and
 // 1309; below, 30,001 nodes 642 and 575; above, 120,007 nodes of degree 24 at 8
 // lanes a row 1746 and 1486, 180,001 nodes of degree 10 2764 and 2511 us for 102).
-template <int VEC>
+template <int VEC, bool FEW>
 static int power_launch_grid(int32_t n, int nb) {
     static std::mutex mu;
     static std::vector<int> resident;  // per device
@@ -728,7 +760,7 @@ static int power_launch_grid(int32_t n, int nb) {
         int coop = 0;
         RMX_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
         if (!coop) throw CudaError(cudaErrorNotSupported, "cooperative launch not supported");
-        RMX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident[dev], k_power<VEC>, kPowT, 0));
+        RMX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident[dev], k_power<VEC, FEW>, kPowT, 0));
     }
     if (resident[dev] < 1) throw CudaError(cudaErrorLaunchOutOfResources, "power iteration does not fit an SM");
     const int64_t lanes = (int64_t)n * VEC, threads = (int64_t)kPowGrid * num_sms() * kPowT;
@@ -738,13 +770,29 @@ static int power_launch_grid(int32_t n, int nb) {
     return (nb + turns - 1) / turns;
 }
 
+template <int VEC, bool FEW>
+static void launch_power_form(int32_t n, int nb, void **args, cudaStream_t s) {
+    RMX_CUDA(cudaLaunchCooperativeKernel((void *)k_power<VEC, FEW>, dim3(power_launch_grid<VEC, FEW>(n, nb)), dim3(kPowT),
+                                         args, 0, s));
+    RMX_LAUNCHED();
+}
+template <int VEC>
+static void launch_power_grid(int32_t n, int nb, void **args, cudaStream_t s) {
+    if (nb <= kPowFew)
+        launch_power_form<VEC, true>(n, nb, args, s);
+    else
+        launch_power_form<VEC, false>(n, nb, args, s);
+}
+
 // Runs the cluster form if the graph is small enough (false: it is not).
 // *iters (device) is -1 if a row is heavy; then nothing was computed.
 template <int VEC>
 static bool launch_power_cluster(int32_t n, int64_t m, const int64_t *in_off, const int32_t *in_src, const double *in_w,
                                  const double *tw, const uint8_t *dangling, double *p, int *iters, double alpha,
                                  int nb, int64_t heavy_deg, cudaStream_t s) {
-    if (n > kClMaxNodes || m > kClMaxLinks || nb > kClMaxBlocks || (int64_t)n * VEC > (int64_t)nb * kPowT) return false;
+    if (n > kClMaxNodes || m > kClMaxLinks || (nb > kClGroups * kClMaxSize && n + m / 32 > kClMaxCost) ||
+        nb > kClMaxBlocks || (int64_t)n * VEC > (int64_t)nb * kPowT)
+        return false;
     const int nbe = (n + kPowT - 1) / kPowT;
     auto smem_for = [&](int C) {
         return sizeof(double) * ((size_t)n + (size_t)((nbe + C - 1) / C) * kPowT + nb + 2 * (size_t)nbe);
@@ -815,9 +863,7 @@ static int launch_power(int32_t n, int64_t m, const int64_t *in_off, const int32
     void *args[] = {(void *)&in_off, (void *)&in_src, (void *)&in_w,  (void *)&tw,    (void *)&dangling, (void *)&n,
                     (void *)&p,      (void *)&y,      (void *)&parts, (void *)&iters, (void *)&alpha,    (void *)&sp,
                     (void *)&pg,     (void *)&nb};
-    RMX_CUDA(cudaLaunchCooperativeKernel((void *)k_power<VEC>, dim3(power_launch_grid<VEC>(n, nb)), dim3(kPowT), args, 0,
-                                         s));
-    RMX_LAUNCHED();
+    launch_power_grid<VEC>(n, nb, args, s);
     RMX_CUDA(cudaMemcpyAsync(&h, iters, sizeof(int), cudaMemcpyDeviceToHost, s));
     RMX_CUDA(cudaStreamSynchronize(s));
     ar.release(mk);
@@ -841,9 +887,7 @@ static void launch_power_into(int32_t n, int64_t m, const int64_t *in_off, const
     void *args[] = {(void *)&in_off, (void *)&in_src, (void *)&in_w,  (void *)&tw,    (void *)&dangling, (void *)&n,
                     (void *)&p,      (void *)&y,      (void *)&parts, (void *)&iters, (void *)&alpha,    (void *)&sp,
                     (void *)&pg,     (void *)&nb};
-    RMX_CUDA(cudaLaunchCooperativeKernel((void *)k_power<VEC>, dim3(power_launch_grid<VEC>(n, nb)), dim3(kPowT), args, 0,
-                                         s));
-    RMX_LAUNCHED();
+    launch_power_grid<VEC>(n, nb, args, s);
 }
 
 void power_iteration_into(int32_t n, int64_t m, const int64_t *in_off, const int32_t *in_src, const double *in_w,

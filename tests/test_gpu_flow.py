@@ -216,3 +216,17 @@ def test_small_graph_flow_with_hub(built_lib, oracle_mod, hub):
     key = np.unique((src * np.int64(n) + dst)[src != dst])
     src, dst = (key // n).astype(np.int32), (key % n).astype(np.int32)
     assert _flow_error(oracle_mod, src, dst, None, n) <= 1e-12
+
+
+@pytest.mark.parametrize("n,deg", [(4096, 12), (4097, 12), (5000, 2), (5100, 2), (3000, 22), (3100, 22),
+                                   (16384, 6), (16385, 6), (18432, 6), (18433, 6)])
+def test_flow_around_the_bounds_of_its_forms(built_lib, oracle_mod, n, deg):
+    """Either side of the bounds of the one-cluster form: four virtual blocks for each of its blocks, and the cost
+    of nodes and links above that; 256 partial sums, one per thread of a block, and 257; 288, the most that the grid form adds from shared
+    memory, and 289."""
+    rng = np.random.default_rng(n + deg)
+    src, dst = rng.integers(0, n - n // 10, n * deg), rng.integers(0, n, n * deg)
+    src[0], dst[0] = 0, n - 1
+    key = np.unique((src * np.int64(n) + dst)[src != dst])
+    src, dst = (key // n).astype(np.int32), (key % n).astype(np.int32)
+    assert _flow_error(oracle_mod, src, dst, rng.uniform(1, 10, len(src)), n) <= 1e-12
