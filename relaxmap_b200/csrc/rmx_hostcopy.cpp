@@ -1,5 +1,6 @@
 #include "rmx_hostcopy.hpp"
 
+#include <sys/mman.h>
 #include <unistd.h>
 
 #include <algorithm>
@@ -73,6 +74,17 @@ bool is_pageable(const void *p) {
     return at.type == cudaMemoryTypeUnregistered;
 }
 
+// Whether 16 of the array's pages, spread from its first to its last, are all in memory.
+bool resident(const char *p, size_t bytes, size_t page) {
+    constexpr size_t kSamples = 16;
+    for (size_t k = 0; k < kSamples; k++) {
+        const uintptr_t a = reinterpret_cast<uintptr_t>(p) + (bytes - 1) * k / (kSamples - 1);
+        unsigned char in = 0;
+        if (mincore(reinterpret_cast<void *>(a & ~(uintptr_t)(page - 1)), page, &in) != 0 || !(in & 1)) return false;
+    }
+    return true;
+}
+
 int host_threads(size_t bytes, size_t per_thread, size_t most) {
     const size_t hw = std::max(1u, std::thread::hardware_concurrency());
     return (int)std::max<size_t>(1, std::min({most, hw, bytes / per_thread}));
@@ -110,8 +122,9 @@ void upload(void *dst, const void *src, size_t bytes, cudaStream_t s) {
 void download(void *dst, const void *src, size_t bytes, cudaStream_t s) {
     if (bytes == 0) return;
     const int T = bytes < kUseMin ? 1 : host_threads(bytes, size_t(1) << 20, 16);
-    if (T > 1 && is_pageable(dst)) {
-        const size_t page = (size_t)sysconf(_SC_PAGESIZE), pages = (bytes + page - 1) / page;
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    if (T > 1 && is_pageable(dst) && !resident(static_cast<const char *>(dst), bytes, page)) {
+        const size_t pages = (bytes + page - 1) / page;
         char *const p = static_cast<char *>(dst);
         run_parallel(T, [&](int t) {  // a write that changes nothing maps the page
             for (size_t k = pages * t / T; k < pages * (t + 1) / T; k++) __atomic_fetch_or(p + k * page, 0, __ATOMIC_RELAXED);

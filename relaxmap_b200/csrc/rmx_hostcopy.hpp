@@ -16,7 +16,9 @@ void upload(void *dst, const void *src, size_t bytes, cudaStream_t s);
 // Device to host on stream s. Pages of a fresh array that have not been touched
 // are first touched by up to 16 threads: faulted in one by one under the copy
 // they took 11.6 of 15.6 ms for 68 MB, by 16 threads 2.1 ms (and 9.5 ms with
-// MADV_POPULATE_WRITE, whose callers wait for one another).
+// MADV_POPULATE_WRITE, whose callers wait for one another). An array that the
+// caller uses again has its pages: starting threads for it only cost time (15 MB
+// 1.12 ms, 0.78 without, which a look at 16 of its pages does not change).
 void download(void *dst, const void *src, size_t bytes, cudaStream_t s);
 
 // Frees the pinned ring (it is allocated again when next needed).

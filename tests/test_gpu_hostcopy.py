@@ -50,3 +50,23 @@ def test_two_threads(built_lib):
     for x in t:
         x.join()
     assert not errors
+
+
+@pytest.mark.parametrize("touched", ["none", "half", "all", "last"])
+def test_results_into_pages_of_an_array(built_lib, touched):
+    """The gradient written to a mapping of which no page, half of the pages, every page or only the last one has
+    been touched, from an address inside a page, equals the one written to pinned memory."""
+    import mmap
+    import torch
+    from relaxmap_b200 import Graph
+    n, src, dst, w = _edges(1 << 20, 5)
+    part = (np.arange(n) // 64).astype(np.int32)
+    with Graph.from_edges(src, dst, w, n=n) as g:
+        want = torch.empty(g.n_links, dtype=torch.float64).pin_memory().numpy()
+        g.adjoint_backward(part, out=want)
+        m = mmap.mmap(-1, 8 * g.n_links + 4096)
+        out = np.frombuffer(m, dtype=np.float64, count=g.n_links, offset=2008)
+        k = {"none": (0, 0), "half": (0, len(out) // 2), "all": (0, len(out)), "last": (len(out) - 1, len(out))}[touched]
+        out[k[0]:k[1]] = 1.0
+        g.adjoint_backward(part, out=out)
+    assert np.array_equal(out, want)
