@@ -14,9 +14,9 @@
 
 namespace rmx {
 
-// job(t) for t < T on T host threads (inline for T == 1); the first exception
-// a job throws (or a failed thread start) is rethrown after every started
-// thread has joined.
+// job(t) for t < T on T host threads (inline for T == 1; the caller also runs
+// the jobs for which no thread could be started); the first exception a job
+// throws is rethrown after every started thread has joined.
 template <typename Job>
 void run_parallel(int T, Job &&job) {
     if (T <= 1) {
@@ -34,12 +34,12 @@ void run_parallel(int T, Job &&job) {
         }
     };
     std::vector<std::thread> pool;
+    int started = 0;
     try {
-        for (int t = 0; t < T; t++) pool.emplace_back(guarded, t);
-    } catch (...) {
-        std::lock_guard<std::mutex> lk(err_mu);
-        if (!err) err = std::current_exception();
+        for (; started < T; started++) pool.emplace_back(guarded, started);
+    } catch (...) {  // the process has all the threads it may have
     }
+    for (int t = started; t < T; t++) guarded(t);
     for (auto &th : pool) th.join();
     if (err) std::rethrow_exception(err);
 }

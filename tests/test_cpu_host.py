@@ -398,3 +398,34 @@ def test_degenerate_files_match_the_oracle(built_lib, oracle_mod, tmp_path):
             ref = {(a, b): x for a, b, x in zip(ld.src.tolist(), ld.dst.tolist(), ld.w.tolist()) if a != b}
             assert acc == ref, name
     assert len(big) > (1 << 20)
+
+
+@pytest.mark.parametrize("allowed", [0, 1, 3, 8])
+def test_jobs_without_a_thread_run_on_the_caller(tmp_path, allowed):
+    """Where the process may start fewer threads than a call wants (here pthread_create fails after the first few),
+    every job is still done, once."""
+    import subprocess
+    (tmp_path / "jobs.cpp").write_text("""
+#include <dlfcn.h>
+#include <pthread.h>
+#include <atomic>
+#include <cerrno>
+#include <cstdio>
+#include "rmx_io.hpp"
+static int allowed = ALLOWED;
+extern "C" int pthread_create(pthread_t *t, const pthread_attr_t *a, void *(*f)(void *), void *x) noexcept {
+    if (allowed-- <= 0) return EAGAIN;
+    using fn = int (*)(pthread_t *, const pthread_attr_t *, void *(*)(void *), void *);
+    return reinterpret_cast<fn>(dlsym(RTLD_NEXT, "pthread_create"))(t, a, f, x);
+}
+int main() {
+    std::atomic<int> ran[8] = {};
+    rmx::run_parallel(8, [&](int t) { ran[t]++; });
+    for (auto &r : ran) printf("%d", r.load());
+}
+""".replace("ALLOWED", str(allowed)))
+    subprocess.run(["g++", "-std=c++17", "-O1", "-rdynamic", "-I", str(ROOT / "relaxmap_b200" / "csrc"), "-I",
+                    str(ROOT / "include"), str(tmp_path / "jobs.cpp"), "-o", str(tmp_path / "jobs"), "-lpthread",
+                    "-ldl"], check=True)
+    r = subprocess.run([str(tmp_path / "jobs")], capture_output=True, text=True)
+    assert (r.returncode, r.stdout) == (0, "11111111"), r.stderr
