@@ -63,11 +63,11 @@ __global__ void k_group_of_nodes(int32_t n, const int32_t *mod, const int64_t *s
 // The groups whose links are to be summed: units of instances that have stopped
 // get none (-1). They keep their modules, are not evaluated again and take part
 // in no later conversion of this superstep, and every superstep starts from the
-// node links, so their links are never needed.
-__global__ void k_group_live(int32_t n, const int32_t *mod, const int64_t *snid, const int32_t *inst,
-                             const uint8_t *live, int32_t *group) {
+// node links, so their links are never needed. sn: every unit's super-node; group
+// may be the same array.
+__global__ void k_group_live(int32_t n, const int32_t *sn, const int32_t *inst, const uint8_t *live, int32_t *group) {
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x)
-        group[v] = live[inst[v]] ? (int32_t)snid[mod[v]] : -1;
+        group[v] = live[inst[v]] ? sn[v] : -1;
 }
 
 __global__ void k_project(int32_t n, const int32_t *node_sn, const int32_t *sn_mod, int32_t *nmod) {
@@ -1278,20 +1278,21 @@ void rmx_graph::convert_to_supernodes(bool from_sn) {
     k_sn_from_modules<<<blocks_for(N, 256, num_sms() * 32), 256, 0, stream>>>(
         N, mods.count, snid, mods.stat, K > 1 ? mods.inst : nullptr, dst.mod, dst.attr, dst.nnodes, dst.inst);
     RMX_LAUNCHED();
-    int32_t *group = nullptr;
-    if (K > 1) {
-        const int32_t n = from_sn ? src.n : N;
-        group = scratch.alloc<int32_t>(std::max(n, 1));
-        k_group_live<<<blocks_for(n, 256, num_sms() * 32), 256, 0, stream>>>(
-            n, from_sn ? src.mod : nmod, snid, from_sn ? src.inst : node_inst, live, group);
-        RMX_LAUNCHED();
-    } else if (from_sn) {
+    k_group_of_nodes<<<blocks_for(N, 256, num_sms() * 32), 256, 0, stream>>>(N, nmod, snid, node_sn);
+    RMX_LAUNCHED();
+    int32_t *group = node_sn;
+    if (from_sn) {
         group = scratch.alloc<int32_t>(std::max(src.n, 1));
         k_group_of_nodes<<<blocks_for(src.n, 256, num_sms() * 32), 256, 0, stream>>>(src.n, src.mod, snid, group);
         RMX_LAUNCHED();
     }
-    k_group_of_nodes<<<blocks_for(N, 256, num_sms() * 32), 256, 0, stream>>>(N, nmod, snid, node_sn);
-    RMX_LAUNCHED();
+    if (K > 1) {  // the nodes' groups take the place of snid, which is not read again: no more scratch than one graph
+        const int32_t n = from_sn ? src.n : N, *const all = group;
+        if (!from_sn) group = reinterpret_cast<int32_t *>(snid);
+        k_group_live<<<blocks_for(n, 256, num_sms() * 32), 256, 0, stream>>>(
+            n, all, from_sn ? src.inst : node_inst, live, group);
+        RMX_LAUNCHED();
+    }
     RMX_CUDA(cudaStreamSynchronize(stream));
     dst.n = (int32_t)nsn;
     if (from_sn)
@@ -1299,7 +1300,7 @@ void rmx_graph::convert_to_supernodes(bool from_sn) {
                                 dst.out_dst, dst.out_fx, dst.out_src, dst.in_off, dst.in_src, dst.in_fx, nullptr,
                                 agg_arena, agg_tab, agg_cap, scratch, stream, &work);
     else
-        dst.m = aggregate_links(N, out_off, out_dst, out_fx, node_lv.out_src, group ? group : node_sn, dst.n, dst.out_off, dst.out_dst,
+        dst.m = aggregate_links(N, out_off, out_dst, out_fx, node_lv.out_src, group, dst.n, dst.out_off, dst.out_dst,
                                 dst.out_fx, dst.out_src, dst.in_off, dst.in_src, dst.in_fx, nullptr, agg_arena, agg_tab,
                                 agg_cap, scratch, stream, &work);
     scratch.release(mk);
@@ -1412,11 +1413,12 @@ void rmx_graph::generate_sub_modules() {
     RMX_LAUNCHED();
     {
         fx_t *rowsum = scratch.alloc<fx_t>(std::max<int64_t>(nsn, 1));
-        int32_t *group = node_sn;
-        if (K > 1) {
-            group = scratch.alloc<int32_t>(N);
-            k_group_live<<<blocks_for(N, 256, num_sms() * 32), 256, 0, stream>>>(N, submod, snid, node_inst, lv, group);
+        const int32_t *group = node_sn;
+        if (K > 1) {  // in the place of snid, which is not read again
+            int32_t *const g = reinterpret_cast<int32_t *>(snid);
+            k_group_live<<<blocks_for(N, 256, num_sms() * 32), 256, 0, stream>>>(N, node_sn, node_inst, lv, g);
             RMX_LAUNCHED();
+            group = g;
         }
         sl.m = aggregate_links(N, out_off, out_dst, out_fx, node_lv.out_src, group, sl.n, sl.out_off, sl.out_dst,
                                sl.out_fx, sl.out_src, sl.in_off, sl.in_src, sl.in_fx, rowsum, agg_arena, agg_tab, agg_cap,

@@ -137,3 +137,33 @@ def test_union_flow_of_uneven_graphs(built_lib, attempts):
     for (n, src, dst, w), part, L in zip(graphs, r["part"], r["L"]):
         with Graph.from_edges(src, dst, w, n=n) as g:
             assert abs(g.codelength(part) - L) <= 1e-10
+
+
+@pytest.fixture
+def every_unit_a_hub():
+    """Every unit of more than 32 links in the hub bin: levels that have one take the separate kernels and their
+    captured loops, as levels of large networks do."""
+    from relaxmap_b200 import get_tuning, set_tuning
+    before = get_tuning()
+    set_tuning(warp_max_degree=32, mid_max_degree=32, block_max_degree=32, large_max_degree=32)
+    yield
+    set_tuning(**before)
+
+
+def test_union_of_many_nodes_and_few_links(built_lib, every_unit_a_hub):
+    """Two graphs of 920,000 nodes, most of them without links, whose conversions by the separate kernels take
+    nearly all of the union's scratch memory, which one graph's conversions would."""
+    from relaxmap_b200 import Batch
+    n, linked = 920_000, 5000
+    gs = []
+    for seed in (1, 2):
+        rng = np.random.default_rng(seed)
+        s = rng.integers(0, linked, 5 * linked)
+        d = np.where(rng.random(len(s)) < 0.8, s // 25 * 25 + rng.integers(0, 25, len(s)), rng.integers(0, linked, len(s)))
+        s, d = np.concatenate([s, np.zeros(40, np.int64)]), np.concatenate([d, np.arange(1, 41)])
+        key = np.unique((s * n + d)[s != d])
+        gs.append((n, (key // n).astype(np.int32), (key % n).astype(np.int32), None))
+    with Batch(gs) as B:
+        r = B.optimize(seed=1, threshold=1e-9)
+    for g, part, L in zip(gs, r["part"], r["L"]):
+        assert abs(_single_L(g, part) - L) <= 1e-10 * L
