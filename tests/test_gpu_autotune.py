@@ -91,3 +91,26 @@ def test_bounds_changed_during_runs(graph):
     finally:
         stop.set()
         t.join()
+
+
+def test_grid_caps_of_the_separate_kernels(built_lib):
+    """Networks with hub units run their node levels as separate kernels, whose grids the caps bound: one block per
+    SM, and many, give the same result on direct launches (a handle's first run) and on captured loops."""
+    from relaxmap_b200 import Graph, TUNING_FIELDS, get_tuning, set_tuning
+    from relaxmap_b200.autotune import DEFAULTS
+    from test_gpu_optimize import hub_network
+    n, src, dst, w = hub_network()
+    before = get_tuning()
+    results = []
+    try:
+        for cfg in (DEFAULTS, dict(DEFAULTS, **{f: 1 for f in TUNING_FIELDS if f.endswith("_grid")}),
+                    dict(DEFAULTS, eval_mid_grid=16, eval_block_grid=8, eval_large_grid=3, eval_warp_grid=8,
+                         eval_reg_grid=16)):
+            set_tuning(**cfg)
+            with Graph.from_edges(src, dst, w, n=n) as G:
+                results += [G.optimize(seed=3) for _ in range(2)]
+    finally:
+        set_tuning(**before)
+    for r in results[1:]:
+        assert r["L"] == results[0]["L"]
+        np.testing.assert_array_equal(r["part"], results[0]["part"])

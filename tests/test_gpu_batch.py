@@ -167,3 +167,37 @@ def test_union_of_many_nodes_and_few_links(built_lib, every_unit_a_hub):
         r = B.optimize(seed=1, threshold=1e-9)
     for g, part, L in zip(gs, r["part"], r["L"]):
         assert abs(_single_L(g, part) - L) <= 1e-10 * L
+
+
+def _launches():
+    from relaxmap_b200 import Graph
+    with Graph.from_edges(np.array([0]), np.array([1]), None, n=2) as G:
+        return G.profile()["kernel_launches"]
+
+
+def _batch_run(gs, **opts):
+    from relaxmap_b200 import Batch
+    with Batch(gs) as B:
+        before = _launches()
+        r = B.optimize(**opts)
+        return r, _launches() - before
+
+
+def _assert_same(a, b):
+    np.testing.assert_array_equal(a["L"], b["L"])
+    np.testing.assert_array_equal(a["best_attempt"], b["best_attempt"])
+    for pa, pb in zip(a["part"], b["part"]):
+        np.testing.assert_array_equal(pa, pb)
+
+
+@pytest.mark.parametrize("prior", [1, 0])
+def test_captured_loops_of_a_union_match_host_loops(built_lib, every_unit_a_hub, capfd, prior):
+    """Levels with hub units run their stages and the coarse-tune sub-problems as captured while graphs, every
+    instance under its own stop rule; per-sweep printing drives the same loops from the host. The captured sweep
+    launches the kernel of every bin, the host loop those of bins with units: more launches show the graph ran."""
+    gs = _graphs()
+    a, captured = _batch_run(gs, seed=2, attempts=3, prior=prior)
+    b, host = _batch_run(gs, seed=2, attempts=3, prior=prior, verbose=2)
+    capfd.readouterr()
+    assert captured > host
+    _assert_same(a, b)

@@ -113,3 +113,45 @@ def test_captured_stage_loops_match_host_loops(built_lib, prior):
             assert r["L"] == ref["L"]
             np.testing.assert_array_equal(r["steps_bits"], ref["steps_bits"])
             assert G.profile()["sweeps"] - s0 == ref_sweeps
+
+
+def hub_network():
+    """30,000 nodes, three of them with 5000 links: its node levels run as separate kernels."""
+    n, hubs = 30_000, 3
+    rng = np.random.default_rng(5)
+    a = rng.integers(hubs, n, 10 * n)
+    b = np.where(rng.random(len(a)) < 0.7, hubs + (a - hubs) // 40 * 40 + rng.integers(0, 40, len(a)),
+                 rng.integers(hubs, n, len(a)))
+    src, dst = [a], [np.minimum(b, n - 1)]
+    for u in range(hubs):  # out- and in-links, 5000 in all
+        other = hubs + rng.permutation(n - hubs)[:5000]
+        src += [np.full(2500, u), other[2500:]]
+        dst += [other[:2500], np.full(2500, u)]
+    src, dst = np.concatenate(src), np.concatenate(dst)
+    key = np.unique((src * n + dst)[src != dst])
+    return n, key // n, key % n, rng.uniform(1, 5, len(key))
+
+
+@pytest.mark.parametrize("prior", [1, 0])
+def test_captured_stage_loops_of_levels_with_hubs(built_lib, prior, capfd):
+    """The node levels of this network have units of more than 4096 links, so their stages run as captured while
+    graphs from the handle's second run on; the first run, and one with per-sweep printing, drive them from the
+    host. Same partition, code length, per-superstep code lengths and number of sweeps. A captured sweep launches
+    the kernel of every bin, the first run's those of bins with units: more launches show that graphs ran."""
+    from relaxmap_b200 import Graph
+    n, src, dst, w = hub_network()
+    runs = []
+    with Graph.from_edges(src, dst, w, n=n) as G:
+        for verbose in (0, 0, 0, 2):
+            before = G.profile()
+            r = G.optimize(seed=4, prior=prior, verbose=verbose)
+            after = G.profile()
+            r["sweeps"] = after["sweeps"] - before["sweeps"]
+            r["launches"] = after["kernel_launches"] - before["kernel_launches"]
+            runs.append(r)
+    capfd.readouterr()
+    for r in runs[1:]:
+        np.testing.assert_array_equal(r["part"], runs[0]["part"])
+        assert r["L"] == runs[0]["L"] and r["sweeps"] == runs[0]["sweeps"]
+        np.testing.assert_array_equal(r["steps_bits"], runs[0]["steps_bits"])
+    assert runs[1]["launches"] == runs[2]["launches"] > runs[0]["launches"]
