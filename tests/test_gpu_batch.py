@@ -201,3 +201,24 @@ def test_captured_loops_of_a_union_match_host_loops(built_lib, every_unit_a_hub,
     capfd.readouterr()
     assert captured > host
     _assert_same(a, b)
+
+
+@pytest.mark.parametrize("prior", [1, 0])
+def test_conversions_of_a_union_with_stopped_instances(built_lib, capfd, prior):
+    """The separate kernels' conversions leave out the links of instances that have stopped, the one-launch
+    conversion sums them all: same partitions, code lengths and best attempts, over graphs from 200 to 6000 nodes
+    that stop after different numbers of supersteps."""
+    from relaxmap_b200 import get_tuning, set_tuning, synth
+    gs = _graphs()
+    for k, spec in enumerate(synth.batched_graphs(5, seed=8, n_range=(2000, 6000), mu_range=(0.1, 0.6))):
+        g = synth.batched_graph(spec)
+        gs.append((g.n, g.src, g.dst, g.w))
+    a, one = _batch_run(gs, seed=4, attempts=3, prior=prior)
+    before = get_tuning()
+    set_tuning(warp_max_degree=32, mid_max_degree=32, block_max_degree=32, large_max_degree=32)
+    try:
+        b, many = _batch_run(gs, seed=4, attempts=3, prior=prior)
+    finally:
+        set_tuning(**before)
+    assert many > 10 * one
+    _assert_same(a, b)
