@@ -1070,15 +1070,17 @@ void rmx_graph::stage_sweeps(Level &lv, bool allow_new, std::vector<double> &L, 
 // evaluation lasts long enough that its 16 warps per SM lose more against the
 // separate kernels' 32 than their launches cost (planted graphs, whole runs: 4.75
 // million links 75 ms as one launch against 80 ms, 7.6 million 157 against 159,
-// 11.4 million 307 against 304, 19 million 293 against 275). A union of
-// instances keeps to one launch: its instances stop one by one, so most of its
-// sweeps are short (160 copies, 27 million links: 217 against 255 ms).
+// 11.4 million 307 against 304, 19 million 293 against 275). Unions of instances
+// too, though their instances stop one by one: 12 copies of one graph, 11.7
+// million links 138 against 132 ms, 40 copies, 39 million 377 against 318, 160
+// copies of 40 graphs, 28 million 135 against 134, 320 copies of 20, 57 million
+// 199 against 175; 32 copies of 8, 6.9 million 25.9 and 25.9.
 constexpr int64_t kFusedMaxLinks = 1 << 23;
 
 // A stage runs as one cooperative launch on levels without hub units and of
 // moderate size, never with profiling events or per-sweep printing.
 bool rmx_graph::fused_ok(const Level &lv) const {
-    return level_hubs == 0 && (K > 1 || lv.m <= kFusedMaxLinks) && !timers.on && opt.verbose < 2 && lv.n > 0 &&
+    return level_hubs == 0 && lv.m <= kFusedMaxLinks && !timers.on && opt.verbose < 2 && lv.n > 0 &&
            scratch.cap - scratch.mark() >= fused_stage_bytes(lv.n);
 }
 

@@ -222,3 +222,17 @@ def test_conversions_of_a_union_with_stopped_instances(built_lib, capfd, prior):
         set_tuning(**before)
     assert many > 10 * one
     _assert_same(a, b)
+
+
+def test_union_above_the_bound_of_the_one_launch_stage(built_lib, capfd):
+    """A union of more than 2^23 links runs its stages at that size as captured while graphs (1087 launches in all,
+    352 with one launch per stage): the same result as the host loops."""
+    from relaxmap_b200 import synth
+    g = synth.planted_partition(40_000, 20, 400, 20, 500, 0.3, seed=5, weights="uniform")
+    assert 11 * g.m > 1 << 23
+    a, captured = _batch_run([(g.n, g.src, g.dst, g.w)], seed=6, attempts=11)
+    b, _ = _batch_run([(g.n, g.src, g.dst, g.w)], seed=6, attempts=11, verbose=2)
+    capfd.readouterr()
+    assert captured > 700
+    _assert_same(a, b)
+    assert abs(_single_L((g.n, g.src, g.dst, g.w), a["part"][0]) - a["L"][0]) <= 1e-10 * a["L"][0]
