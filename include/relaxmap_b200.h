@@ -300,9 +300,13 @@ rmx_status rmx_adjoint_backward(rmx_graph *g, const int32_t *part, double tau, d
  * partitioned by module into ceil(links / hub_partition_links) parts, each
  * aggregated by one block (so are the links of a super-node of more than
  * 16384 member links when the coarsening sums them). Results do not depend on
- * these values (every bin's kernel loops over its units by grid stride,
- * module statistics are exact integer sums, and every bin computes the same
- * change per candidate), only the time does. rmx_set_tuning takes effect at
+ * the grid caps (every bin's kernel loops over its units by grid stride, and
+ * module statistics are exact integer sums), only the time does. The degree
+ * bounds assign units to kernels that compute the same change per candidate,
+ * but for the last bit of its rounding in the hub bin: only a tie exact to that
+ * bit could fall the other way. Levels without hub units and of up to 2^23
+ * links run each stage of sweeps as one launch, which goes by the degree bounds
+ * and has no use for the grid caps. rmx_set_tuning takes effect at
  * the next stage of sweeps, also of a run in progress on another thread, which
  * reads all values at once when a stage begins; sweep pipelines captured as CUDA graphs under other values
  * are captured again. Each grid cap must lie in [1, 64], and
@@ -328,7 +332,11 @@ typedef struct rmx_tuning {
 rmx_status rmx_get_tuning(rmx_tuning *out);
 rmx_status rmx_set_tuning(const rmx_tuning *t);
 
-/* Device-time profiling of the handle's kernels (CUDA events on its stream). */
+/* Device-time profiling of the handle's kernels (CUDA events on its stream).
+ * Profiled runs launch every kernel from the host between events, also on the
+ * levels whose stages otherwise run as one launch or as a captured loop: the
+ * results are the same, the times those of the separate kernels, so a run takes
+ * longer than without (most of all on small graphs). */
 rmx_status rmx_set_profiling(rmx_graph *g, int32_t on);
 rmx_status rmx_get_profile(const rmx_graph *g, rmx_profile *out);
 

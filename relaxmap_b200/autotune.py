@@ -1,10 +1,13 @@
 """Autotuner for the launch shape of move evaluation (rmx_set_tuning).
 
 The grid cap of each degree bin (blocks per SM) and the degree bounds that
-assign units to the bins change the time of an optimiser run, never its
-result: every evaluation kernel loops over its bin's units by grid stride,
-module statistics are exact integer sums, and every bin computes the same
-change per candidate. The tuner
+assign units to the bins are there to change the time of an optimiser run, not
+its result: every evaluation kernel loops over its bin's units by grid stride,
+module statistics are exact integer sums, and the bins compute the same change
+per candidate (up to the last bit of its rounding in the hub bin). The grid caps
+act on levels with hub units or of more than 2^23 links; other levels run a
+stage as one launch, whose time only the degree bounds change, so tune on a graph
+of the size and kind that is to be optimised. The tuner
 times full runs of a representative graph under candidate caps, one knob at a
 time (coordinate descent, a few passes), keeps a candidate only when it is
 faster by more than the noise margin, and checks that every candidate

@@ -6,7 +6,7 @@
 // packed into waves; a wave is ONE disjoint-union graph on the device whose
 // components (graph-attempt copies) are independent instances of the engine:
 // every stop rule of the superstep loop is applied per instance, the flow is
-// computed once per graph (one block per graph) and shared by its copies, and
+// computed once per graph (all graphs' rows by one grid) and shared by its copies, and
 // all instances advance in the same kernel launches. Copies of a graph differ
 // in their random choices (sub-batch assignment and empty-module bids hash
 // the unit id), as attempts with different seeds do. The best attempt of every

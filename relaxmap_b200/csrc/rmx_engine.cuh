@@ -180,10 +180,11 @@ struct Timers {
 // (SweepWork::tune):
 // the grid cap of each bin in blocks per SM, and the degree bounds that
 // assign units to the warp, mid, block and large bins (units above large_max
-// go to the hub bin). Results do not depend on them (each bin's kernel loops
-// over its units by grid stride, every bin computes the same exact integer
-// sums and the same change per candidate), only the time does. The hub bin's
-// grid is not tuned: its global table slices are indexed by block.
+// go to the hub bin). Results do not depend on the caps (each bin's kernel loops
+// over its units by grid stride and computes exact integer sums), only the time
+// does; the hub bin rounds the change of a candidate differently in the last bit
+// (make_ctx), so a bound could turn a tie that is exact to that bit. The hub bin's
+// grids are not tuned. A stage run as one launch goes by the bounds alone.
 struct EvalTuning {
     int mid, block, large, warp, reg;              // grid caps
     int warp_max, mid_max, block_max, large_max;   // degree bounds (at most 128, 512, 1024, 4096)

@@ -339,9 +339,9 @@ struct PowSplit {
 };
 
 // The flow vector's gathered copy: on graphs whose flow vector is larger
-// than L2 the pull gathers from a copy holding only the nodes that have
-// out-links (rank[i] >= 0: node i's place in it; gsrc: in_src renumbered to
-// those places), small enough to stay in L2. Values are the same doubles,
+// than about half of L2 (gather_copy has the rule) the pull gathers from a copy
+// holding only the nodes that have out-links (rank[i] >= 0: node i's place in it;
+// gsrc: in_src renumbered to those places), of which more stays in L2. Values are the same doubles,
 // so the sums are unchanged.
 struct PowGather {
     const int32_t *gsrc = nullptr;  // nullptr: gather from x itself

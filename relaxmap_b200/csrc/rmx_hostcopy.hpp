@@ -6,7 +6,8 @@
 
 namespace rmx {
 
-// Host to device on stream s; src may be reused when the call returns. Large
+// Host to device on stream s. A pageable src may be reused when the call returns;
+// a pinned one is read by the device until the stream has passed the copy. Large
 // pageable arrays go through a pinned ring filled by several threads: the
 // driver's own staging copies them on one (90 MB: 8.4 ms; with the endpoint
 // check on eight threads too, creating a handle from 5.67 million weighted edges
