@@ -576,7 +576,10 @@ void rmx_graph::create(const int32_t *src, const int32_t *dst, const double *w, 
     configure_eval_kernels();
     // input edges, and an upper bound on the kept links of the whole union
     const int64_t Ein = std::max<int64_t>(n_edges, 1), Eb = std::max<int64_t>(repl ? u->full_edges : n_edges, 1);
-    scratch.init((size_t)(88 * Eb + 24 * (int64_t)n + 40 * (int64_t)K) + (64u << 20));
+    // a union's build holds the input and the canonical copies' CSR and CSC (40 bytes per edge) beside build_csr's
+    // scratch (54), which is more than the other uses where every copy is canonical (one attempt)
+    const int64_t build = repl ? 96 * Ein : 0;
+    scratch.init((size_t)(std::max(88 * Eb, build) + 24 * (int64_t)n + 40 * (int64_t)K) + (64u << 20));
     // long-lived arrays: node CSR/CSC, three levels, module and instance state
     perm.init((size_t)(156 * Eb + 696 * (int64_t)n + (K > 1 ? 16 * (int64_t)n + 64 * (int64_t)K : 0)) + (64u << 20));
     out_off = perm.alloc<int64_t>(n + 1);

@@ -236,3 +236,19 @@ def test_union_above_the_bound_of_the_one_launch_stage(built_lib, capfd):
     assert captured > 700
     _assert_same(a, b)
     assert abs(_single_L((g.n, g.src, g.dst, g.w), a["part"][0]) - a["L"][0]) <= 1e-10 * a["L"][0]
+
+
+def test_union_of_large_graphs_with_one_attempt(built_lib):
+    """Every copy of the union is canonical: the build's scratch, with the input and the copies' links in it, is the
+    union's largest."""
+    n, m = 400_000, 9_000_000  # hardly an edge twice
+    gs = []
+    for seed in (1, 2):
+        rng = np.random.default_rng(seed)
+        s, d = rng.integers(0, n, m), rng.integers(0, n, m)
+        near = rng.random(m) < 0.7
+        d[near] = s[near] // 1000 * 1000 + rng.integers(0, 1000, int(near.sum()))
+        gs.append((n, s.astype(np.int32), d.astype(np.int32), None))
+    r, _ = _batch_run(gs, seed=1, attempts=1, max_iter=1)
+    for g, part, L in zip(gs, r["part"], r["L"]):
+        assert abs(_single_L(g, part) - L) <= 1e-10 * L
