@@ -571,6 +571,8 @@ void rmx_graph::create(const int32_t *src, const int32_t *dst, const double *w, 
         K = u->K;
         inst_noff.assign(u->inst_noff, u->inst_noff + K + 1);
         inst_canon.assign(u->inst_canon, u->inst_canon + K);
+        n_canon = 0;
+        for (int32_t k = 0; k < K; k++) n_canon += inst_canon[k] == k;
     }
     RMX_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     configure_eval_kernels();
@@ -1073,17 +1075,21 @@ void rmx_graph::stage_sweeps(Level &lv, bool allow_new, std::vector<double> &L, 
 // evaluation lasts long enough that its 16 warps per SM lose more against the
 // separate kernels' 32 than their launches cost (planted graphs, whole runs: 4.75
 // million links 75 ms as one launch against 80 ms, 7.6 million 157 against 159,
-// 11.4 million 307 against 304, 19 million 293 against 275). Unions of instances
-// too, though their instances stop one by one: 12 copies of one graph, 11.7
-// million links 138 against 132 ms, 40 copies, 39 million 377 against 318, 160
-// copies of 40 graphs, 28 million 135 against 134, 320 copies of 20, 57 million
-// 199 against 175; 32 copies of 8, 6.9 million 25.9 and 25.9.
-constexpr int64_t kFusedMaxLinks = 1 << 23;
+// 11.4 million 307 against 304, 19 million 293 against 275). Copies of one graph
+// stop at about the same time and have nearly the same bound, the captured graphs'
+// cost for a handle that runs once included (50 copies, 9.5 million links, 84
+// against 88 ms a call, 10 of a larger one, 9.8 million, 126 against 127; 12, 11.7
+// million, 151 against 149, 20, 19.6 million, 202 against 183). In a union of graphs of
+// different sizes the largest go on long after the others, in sweeps that are
+// short for the number of links: 40 graphs x 4, 28 million links, 178 against 182
+// ms, 45 x 4, 31 million, 219 against 225; 50 x 4, 36 million, 205 against 201.
+constexpr int64_t kFusedMaxLinks = 1 << 23, kFusedMaxCopyLinks = 10 << 20, kFusedMaxUnionLinks = 1 << 25;
 
 // A stage runs as one cooperative launch on levels without hub units and of
 // moderate size, never with profiling events or per-sweep printing.
 bool rmx_graph::fused_ok(const Level &lv) const {
-    return level_hubs == 0 && lv.m <= kFusedMaxLinks && !timers.on && opt.verbose < 2 && lv.n > 0 &&
+    const int64_t most = K == 1 ? kFusedMaxLinks : n_canon == 1 ? kFusedMaxCopyLinks : kFusedMaxUnionLinks;
+    return level_hubs == 0 && lv.m <= most && !timers.on && opt.verbose < 2 && lv.n > 0 &&
            scratch.cap - scratch.mark() >= fused_stage_bytes(lv.n);
 }
 

@@ -125,6 +125,7 @@ struct rmx_graph {
     uint8_t *live = nullptr;            // device: instances whose links the next conversion sums (K > 1)
     std::vector<int64_t> inst_noff;     // host, K + 1
     std::vector<int32_t> inst_canon;    // host: the copy whose flow instance k shares (itself if first)
+    int32_t n_canon = 1;                // different graphs among them
     std::vector<double> L0v;            // initial code length per instance
 
     // ---- CUDA graphs of the sweep pipeline (off: every kernel launched directly)

@@ -224,18 +224,28 @@ def test_conversions_of_a_union_with_stopped_instances(built_lib, capfd, prior):
     _assert_same(a, b)
 
 
-def test_union_above_the_bound_of_the_one_launch_stage(built_lib, capfd):
-    """A union of more than 2^23 links runs its stages at that size as captured while graphs (1087 launches in all,
-    352 with one launch per stage): the same result as the host loops."""
+@pytest.mark.parametrize("graphs,below,bound", [(1, 13, 10 << 20), (2, 21, 1 << 25)])
+def test_union_around_the_bounds_of_the_one_launch_stage(built_lib, capfd, graphs, below, bound):
+    """Copies of one graph have their stages run as one launch up to 10 * 2^20 links, unions of several up to 2^25;
+    one attempt more and they run as captured while graphs, with far more launches: the same result as the host
+    loops on either side."""
     from relaxmap_b200 import synth
-    g = synth.planted_partition(40_000, 20, 400, 20, 500, 0.3, seed=5, weights="uniform")
-    assert 11 * g.m > 1 << 23
-    a, captured = _batch_run([(g.n, g.src, g.dst, g.w)], seed=6, attempts=11)
-    b, _ = _batch_run([(g.n, g.src, g.dst, g.w)], seed=6, attempts=11, verbose=2)
+    gs = []
+    for seed in range(graphs):
+        g = synth.planted_partition(40_000, 20, 400, 20, 500, 0.3, seed=5 + seed, weights="uniform")
+        gs.append((g.n, g.src, g.dst, g.w))
+    links = sum(len(g[1]) for g in gs)
+    assert below * links <= bound < (below + 1) * links
+    launches = []
+    for attempts in (below, below + 1):
+        a, n = _batch_run(gs, seed=6, attempts=attempts, max_iter=3)
+        b, _ = _batch_run(gs, seed=6, attempts=attempts, max_iter=3, verbose=2)
+        launches.append(n)
+        _assert_same(a, b)
+        for g, part, L in zip(gs, a["part"], a["L"]):
+            assert abs(_single_L(g, part) - L) <= 1e-10 * L
     capfd.readouterr()
-    assert captured > 700
-    _assert_same(a, b)
-    assert abs(_single_L((g.n, g.src, g.dst, g.w), a["part"][0]) - a["L"][0]) <= 1e-10 * a["L"][0]
+    assert launches[1] > launches[0] + 200
 
 
 def test_union_of_large_graphs_with_one_attempt(built_lib):
