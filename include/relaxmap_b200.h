@@ -305,7 +305,8 @@ rmx_status rmx_adjoint_backward(rmx_graph *g, const int32_t *part, double tau, d
  * bounds assign units to kernels that compute the same change per candidate,
  * but for the last bit of its rounding in the hub bin: only a tie exact to that
  * bit could fall the other way. Levels without hub units and of up to 2^23
- * links run each stage of sweeps as one launch, which goes by the degree bounds
+ * links (2^25 in a batch of several graphs, 10 * 2^20 in a batch of copies of
+ * one) run each stage of sweeps as one launch, which goes by the degree bounds
  * and has no use for the grid caps. rmx_set_tuning takes effect at
  * the next stage of sweeps, also of a run in progress on another thread, which
  * reads all values at once when a stage begins; sweep pipelines captured as CUDA graphs under other values

@@ -5,7 +5,7 @@ assign units to the bins are there to change the time of an optimiser run, not
 its result: every evaluation kernel loops over its bin's units by grid stride,
 module statistics are exact integer sums, and the bins compute the same change
 per candidate (up to the last bit of its rounding in the hub bin). The grid caps
-act on levels with hub units or of more than 2^23 links; other levels run a
+act on levels with hub units or of more than 2^23 links (more in a batch); other levels run a
 stage as one launch, whose time only the degree bounds change, so tune on a graph
 of the size and kind that is to be optimised. The tuner
 times full runs of a representative graph under candidate caps, one knob at a

@@ -30,7 +30,8 @@
 // and 10.8 against 6.5 us on a 44-unit level. Measured as whole runs against
 // the kernel pipeline as it was then: 1000 nodes 2.78 -> 1.97 ms, 20,011 nodes in
 // normal mode 19.0 -> 13.0 ms, 150,001 nodes 83 -> 64 ms. Levels of more than
-// 2^23 links are left to that pipeline's kernels of 32 warps per SM.
+// 2^23 links (unions: kFusedMaxUnionLinks in rmx_engine.cu) are left to that
+// pipeline's kernels of 32 warps per SM.
 #include <cooperative_groups.h>
 
 #include <algorithm>
