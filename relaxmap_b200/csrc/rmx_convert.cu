@@ -39,7 +39,7 @@ constexpr int kCvList = 256;             // slots a warp can have filled
 constexpr int kCvIlp = 4;
 // Blocks per SM. With one, larger levels wait on the sums' shared-memory and
 // column atomics: all conversions of a run on 250,001 nodes 15.3 ms, with two
-// (64 registers, no spills) 14.9; on 400,001 nodes 39.1 and 37.9.
+// (64 registers, 68 bytes a thread spilt) 14.9; on 400,001 nodes 39.1 and 37.9.
 constexpr int kCvBlocks = 2;
 // links of a group summed by a warp, four warps, a block in one pass, a block in several
 constexpr int kCvWarpMax = 256, kCvTeamMax = 1024, kCvBlockMax = 4096, kCvMost = 16384;
